@@ -140,6 +140,11 @@ constexpr int kGatherThreads = kTileW * kTileH;
 
 // engine_kernels.cu
 template <typename T> cudaError_t launch_position_pass(const PositionPassArgs<T> &a, int shape, cudaStream_t s);
+// anypass.cu: the shared-memory position pass for any detector whose sides have no prime factor above 31 and whose plane
+// (with an odd pitch) fits one CTA; the pass of every such size without a compile-time plan.
+bool any_pass_applicable(int rows, int columns, bool fp64);
+cudaError_t configure_any_pass();
+template <typename T> cudaError_t launch_any_pass(const PositionPassArgs<T> &a, cudaStream_t s);
 // linepass.cu: the FP32 position pass for 64 x 64 and 96 x 96 detectors with register-resident line transforms (four
 // steps: R-point DFTs in registers, one in-group exchange, G-point DFTs), one CTA per position; the default FP32 pass
 // at those sizes (cubo_ptycho_params.pass_shape 0).

@@ -690,6 +690,8 @@ cudaError_t configure_kernels() {
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
             if (e != cudaSuccess) return e;
         }
+    e = configure_any_pass();
+    if (e != cudaSuccess) return e;
     return configure_line_pass();
 }
 
@@ -737,6 +739,8 @@ cudaError_t launch_position_pass(const PositionPassArgs<T> &a, int shape, cudaSt
     const int threads = a.rows == a.columns ? fixed_threads<T>(a.rows, shape) : 0;
     if (threads > 0)
         fixed_kernel<T>(a.rows, threads)<<<a.count, threads, smem, s>>>(a);
+    else if (any_pass_applicable(a.rows, a.columns, std::is_same<T, double>::value))
+        return launch_any_pass<T>(a, s);
     else
         position_pass_kernel<T, kPassThreads, maxn><<<a.count, kPassThreads, smem, s>>>(a);
     return cudaGetLastError();
