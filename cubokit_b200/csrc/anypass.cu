@@ -11,62 +11,6 @@ namespace {
 
 constexpr size_t kAnySmem = 226 * 1024;  // dynamic shared memory of one CTA: 227 KB less the kernel's static part
 
-// The fewest allowed factors whose product is L, the largest factor as small as possible, ascending; count 0: L has a
-// prime factor above 31 (or does not fit the stages).
-int best_factors(int L, int most, int *out) {
-    static const int radices[] = {2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 19, 23, 29, 31};
-    if (L < 2) return 0;
-    for (int count = 1; count <= kAnyStages; count++) {
-        // factors not above `cap`, the cap raised until the length splits into `count` of them
-        for (int cap : radices) {
-            if (cap > most) break;
-            int f[kAnyStages], rest = L, depth = 0;
-            int at[kAnyStages];  // index of the factor tried at each depth, descending
-            at[0] = (int)(sizeof(radices) / sizeof(radices[0])) - 1;
-            while (depth >= 0) {
-                bool down = false;
-                for (int &i = at[depth]; i >= 0; i--) {
-                    const int r = radices[i];
-                    if (r > cap || rest % r != 0) continue;
-                    f[depth] = r;
-                    if (depth + 1 == count) {
-                        if (rest != r) continue;
-                        for (int k = 0; k < count; k++) out[k] = f[count - 1 - k];  // ascending
-                        return count;
-                    }
-                    rest /= r;
-                    at[depth + 1] = i;
-                    down = true;
-                    break;
-                }
-                if (down) depth++;
-                else {
-                    depth--;
-                    if (depth >= 0) { rest *= f[depth]; at[depth]--; }
-                }
-            }
-        }
-    }
-    return 0;
-}
-
-// Ascending radices give the row ends (stage 1) the longest contiguous runs of global memory; the column lines take them
-// descending, so that the centre step, which holds the amplitudes too, has the smallest.
-bool plan_line(int L, bool ascending, AnyLine *l) {
-    int f[kAnyStages];
-    const int count = best_factors(L, 31, f);
-    if (count == 0) return false;
-    l->L = L;
-    l->stages = count;
-    int sub = L;
-    for (int i = 0; i < count; i++) {
-        l->r[i] = ascending ? f[i] : f[count - 1 - i];
-        sub /= l->r[i];
-        l->sub[i] = divisor(sub);
-    }
-    return true;
-}
-
 template <typename T>
 size_t any_smem(int rows, int columns) {
     const size_t pitch = (size_t)(columns | 1);
@@ -102,7 +46,7 @@ int any_threads(int rows, int columns) {
 
 bool any_pass_applicable(int rows, int columns, bool fp64) {
     AnyLine r, c;
-    if ((long long)rows * columns >= 65536 || !plan_line(rows, false, &r) || !plan_line(columns, true, &c)) return false;
+    if (rows < 2 || columns < 2 || (long long)rows * columns >= 65536 || !plan_line(rows, 31, false, &r) || !plan_line(columns, 31, true, &c)) return false;
     return (fp64 ? any_smem<double>(rows, columns) : any_smem<float>(rows, columns)) <= kAnySmem;
 }
 
@@ -123,7 +67,7 @@ cudaError_t launch_any_pass(const PositionPassArgs<T> &a, cudaStream_t s) {
     if (a.count <= 0) return cudaSuccess;
     AnyPassArgs<T> g{};
     g.p = a;
-    if (!plan_line(a.rows, false, &g.rows) || !plan_line(a.columns, true, &g.columns)) return cudaErrorInvalidValue;
+    if (!plan_line(a.rows, 31, false, &g.rows) || !plan_line(a.columns, 31, true, &g.columns)) return cudaErrorInvalidValue;
     g.by_rows = divisor(a.rows);
     g.by_columns = divisor(a.columns);
     g.pitch = a.columns | 1;

@@ -45,7 +45,8 @@ __device__ __forceinline__ int quotient(int i, const Divisor &v) {
 
 struct AnyLine {
     int L, stages;
-    int r[kAnyStages];    // radix of each stage
+    int r[kAnyStages];        // radix of each stage
+    int before[kAnyStages];   // r_1 .. r_{i-1}
     Divisor sub[kAnyStages];  // L / (r_1 .. r_i)
 };
 
@@ -61,12 +62,11 @@ __device__ __forceinline__ int awrap(int v, int size) { return v < 0 ? v + size 
 
 // The frequency slot e of a transformed line holds: e = sum q_i sub_i, k = sum q_i r_1 .. r_{i-1}.
 static __device__ int slot_frequency(const AnyLine &l, int e) {
-    int k = 0, scale = 1;
+    int k = 0;
     for (int i = 0; i < l.stages; i++) {
         const int q = quotient(e, l.sub[i]);
         e -= q * (int)l.sub[i].d;
-        k += q * scale;
-        scale *= l.r[i];
+        k += q * l.before[i];
     }
     return k;
 }
@@ -79,7 +79,8 @@ __device__ __forceinline__ void twiddle(C2<T> (&x)[R], int j, int step, const C2
     for (int q = 1; q < R; q++) x[q] = regdft::turn<C2<T>, INV>(x[q], tw[q * e]);
 }
 
-// An inner stage of every line: lines `line` apart, samples `elem` apart, stage s of plan l.
+// An inner stage of every line: lines `line` apart, samples `elem` apart, stage s of plan l, whose twiddles are powers of
+// W_B = tw[scale] (B the stage's block).
 template <typename T, bool INV, int R>
 __device__ __forceinline__ void inner_stage(C2<T> *D, const AnyLine &l, int s, int scale, const Divisor &lines,
                                             int line, int elem, const C2<T> *tw) {
@@ -251,21 +252,16 @@ __global__ void __launch_bounds__(kAnyThreads<T>, 1) any_pass_kernel(const __gri
         first_stage<T, decltype(r)::value>(D, g, rr, cc, a.shifted + (size_t)cls * a.n, twc);
     });
     __syncthreads();
-    int scale = g.columns.r[0];
     for (int s = 1; s < g.columns.stages; s++) {
         with_radix<WIDE>(g.columns.r[s], [&](auto r) {
-            inner_stage<T, false, decltype(r)::value>(D, g.columns, s, scale, g.by_rows, g.pitch, 1, twc);
+            inner_stage<T, false, decltype(r)::value>(D, g.columns, s, g.columns.before[s], g.by_rows, g.pitch, 1, twc);
         });
-        scale *= g.columns.r[s];
         __syncthreads();
     }
-    const int column_scale = scale;
-    scale = 1;
     for (int s = 0; s + 1 < g.rows.stages; s++) {
         with_radix<WIDE>(g.rows.r[s], [&](auto r) {
-            inner_stage<T, false, decltype(r)::value>(D, g.rows, s, scale, g.by_columns, 1, g.pitch, twr);
+            inner_stage<T, false, decltype(r)::value>(D, g.rows, s, g.rows.before[s], g.by_columns, 1, g.pitch, twr);
         });
-        scale *= g.rows.r[s];
         __syncthreads();
     }
     double err = 0;
@@ -274,17 +270,14 @@ __global__ void __launch_bounds__(kAnyThreads<T>, 1) any_pass_kernel(const __gri
     });
     __syncthreads();
     for (int s = g.rows.stages - 2; s >= 0; s--) {
-        scale /= g.rows.r[s];
         with_radix<WIDE>(g.rows.r[s], [&](auto r) {
-            inner_stage<T, true, decltype(r)::value>(D, g.rows, s, scale, g.by_columns, 1, g.pitch, twr);
+            inner_stage<T, true, decltype(r)::value>(D, g.rows, s, g.rows.before[s], g.by_columns, 1, g.pitch, twr);
         });
         __syncthreads();
     }
-    scale = column_scale;
     for (int s = g.columns.stages - 1; s >= 1; s--) {
-        scale /= g.columns.r[s];
         with_radix<WIDE>(g.columns.r[s], [&](auto r) {
-            inner_stage<T, true, decltype(r)::value>(D, g.columns, s, scale, g.by_rows, g.pitch, 1, twc);
+            inner_stage<T, true, decltype(r)::value>(D, g.columns, s, g.columns.before[s], g.by_rows, g.pitch, 1, twc);
         });
         __syncthreads();
     }
@@ -301,6 +294,63 @@ __global__ void __launch_bounds__(kAnyThreads<T>, 1) any_pass_kernel(const __gri
         for (int w = 0; w < (int)blockDim.x / 32; w++) total += scratch[w];
         a.error[p] = total;
     }
+}
+
+// The fewest allowed factors whose product is L, the largest factor as small as possible, ascending; count 0: L has a
+// prime factor above 31 (or does not fit the stages).
+inline int best_factors(int L, int most, int *out) {
+    static const int radices[] = {2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 19, 23, 29, 31};
+    if (L < 2) return 0;
+    for (int count = 1; count <= kAnyStages; count++) {
+        // factors not above `cap`, the cap raised until the length splits into `count` of them
+        for (int cap : radices) {
+            if (cap > most) break;
+            int f[kAnyStages], rest = L, depth = 0;
+            int at[kAnyStages];  // index of the factor tried at each depth, descending
+            at[0] = (int)(sizeof(radices) / sizeof(radices[0])) - 1;
+            while (depth >= 0) {
+                bool down = false;
+                for (int &i = at[depth]; i >= 0; i--) {
+                    const int r = radices[i];
+                    if (r > cap || rest % r != 0) continue;
+                    f[depth] = r;
+                    if (depth + 1 == count) {
+                        if (rest != r) continue;
+                        for (int k = 0; k < count; k++) out[k] = f[count - 1 - k];  // ascending
+                        return count;
+                    }
+                    rest /= r;
+                    at[depth + 1] = i;
+                    down = true;
+                    break;
+                }
+                if (down) depth++;
+                else {
+                    depth--;
+                    if (depth >= 0) { rest *= f[depth]; at[depth]--; }
+                }
+            }
+        }
+    }
+    return 0;
+}
+
+// Ascending radices give the row ends (stage 1) the longest contiguous runs of global memory; the column lines take them
+// descending, so that the centre step, which holds the amplitudes too, has the smallest.
+inline bool plan_line(int L, int most, bool ascending, AnyLine *l) {
+    int f[kAnyStages] = {};
+    const int count = L == 1 ? 0 : best_factors(L, most, f);
+    if (count == 0 && L != 1) return false;
+    l->L = L;
+    l->stages = count;
+    int done = 1;
+    for (int i = 0; i < count; i++) {
+        l->r[i] = ascending ? f[i] : f[count - 1 - i];
+        l->before[i] = done;
+        done *= l->r[i];
+        l->sub[i] = divisor(L / done);
+    }
+    return true;
 }
 
 using AnyKernelF = void (*)(AnyPassArgs<float>);

@@ -258,13 +258,13 @@ cudaError_t launch_average_slices(double2 *object, int slices, long long plane, 
 // step -> inverse FFT (unscaled) -> out; kPlaneForward: the input (times the patch) -> FFT -> out, unscaled;
 // kPlaneInverse: a spectrum -> the pointwise step -> inverse FFT (unscaled) -> out.
 enum { kPlaneFull = 0, kPlaneForward = 1, kPlaneInverse = 2 };
-enum { kInputByPosition = 0, kInputByClass = 1, kInputSingle = 2 };
+enum { kInputByPosition = 0, kInputByClass = 1 };
 enum { kPointwiseNone = 0, kPointwiseFactors = 1, kPointwiseProjection = 2, kPointwiseSolve = 3,
        kPointwiseFactorPlane = 4 };
 struct Plane128Args {
     int mode;
     int first, count;
-    const double2 *in;              // input plane of position p: in + (p, scan.cls[p] or 0 by in_kind) * 16384
+    const double2 *in;              // input plane of position p: in + (p, scan.cls[p] by in_kind) * 16384
     int in_kind;
     const double2 *object;          // full / forward: the object patch factor, conjugated when conj_object; null: none
     int conj_object;
@@ -273,9 +273,8 @@ struct Plane128Args {
     int object_rows, object_columns;
     int pointwise;                  // kPointwiseFactors: x prop_rows[kr] prop_columns[kc] x scale; kPointwiseProjection
                                     // (full mode): modulus projection with amplitudes (x inv_n) and error[p]
-    const double2 *prop_rows;       // 128 factors of the row frequency, then prop_stride further per position
+    const double2 *prop_rows;       // 128 factors of the row frequency
     const double2 *prop_columns;    // 128 of the column frequency; both conjugated when conj_prop
-    long long prop_stride;          // (a Fresnel kernel and the Fourier-shift ramps both factor so)
     int conj_prop;
     double scale;
     const float *amplitudes;        // [positions][128 x 128]
@@ -348,6 +347,14 @@ cudaError_t launch_renormalise(double2 *dst, const double2 *src, int n, const do
                                cudaStream_t s);
 cudaError_t launch_support_mask(double2 *probe, const unsigned char *mask, int n, cudaStream_t s);
 cudaError_t launch_magnitude(const double2 *data, double *out, int n, cudaStream_t s);
+// shift.cu: out[f] = ifft2(spectrum x the ramps of class f), FP64 arithmetic, one launch, for the sizes shift_applicable
+// accepts.
+bool shift_applicable(int rows, int columns);
+cudaError_t configure_shift();
+template <typename T>
+cudaError_t launch_shift_table(const Fft2Plan64 &p, const double2 *spectrum, double2 *scratch,
+                               const double2 *ramps_rows, const double2 *ramps_columns, int classes, C2<T> *out,
+                               cudaStream_t s);  // scratch: one plane
 cudaError_t launch_shift_ramps(const double2 *spectrum, const double2 *ramps_rows, const double2 *ramps_columns,
                                int rows, int columns, int classes, double2 *out, cudaStream_t s);
 // The phase ramps of `classes` fractional shifts (dr, dc) = fractions[f]: exp(-2 pi i frequency(k) d) per row and column.

@@ -271,6 +271,7 @@ struct cubo_ptycho_plan {
     DeviceBuffer amplitudes, rr, cc, cls, tile_start, tile_list;
     DeviceBuffer object, grad_o, weight_o, tile_max;
     DeviceBuffer dpsi, error, errors, iteration;
+    bool fused_shift = false;  // the shift table in one launch (shift.cu)
     DeviceBuffer probe64, scratch64, spectrum64, shifted, shift_tmp64, ramps_r64, ramps_c64;
     DeviceBuffer partial_grad, partial_weight, grad_p64, weight_p64, probe_block_max;
     DeviceBuffer maxes, sums, aperture64, mask_dev, error_scratch, loss_slot;
@@ -500,7 +501,7 @@ void build_scan(cubo_ptycho_plan *p, const double *rows_in, const double *column
     if (p->shifted.bytes < shifted_bytes) check(p->shifted.alloc(shifted_bytes), "cudaMalloc");
     const int frac = p->classes - 1;
     if (frac > 0) {
-        if (p->shift_tmp64.bytes < (size_t)frac * n * sizeof(double2))
+        if (!p->fused_shift && p->shift_tmp64.bytes < (size_t)frac * n * sizeof(double2))
             check(p->shift_tmp64.alloc((size_t)frac * n * sizeof(double2)), "cudaMalloc shift table");
         if (p->ramps_r64.bytes < (size_t)frac * R * sizeof(double2))
             check(p->ramps_r64.alloc((size_t)frac * R * sizeof(double2)), "cudaMalloc");
@@ -744,7 +745,7 @@ void enqueue_plane128(cubo_ptycho_plan *p, Kind kind, const double2 *in, bool by
     Plane128Args a = plane_args(p, kPlaneFull);
     a.in = in; a.in_kind = by_class ? kInputByClass : kInputByPosition; a.object = object;
     a.conj_object = conj_object ? 1 : 0; a.pointwise = project ? kPointwiseProjection : kPointwiseFactors;
-    a.prop_rows = prop_factors; a.prop_columns = prop_factors ? prop_factors + 128 : nullptr; a.prop_stride = 0;
+    a.prop_rows = prop_factors; a.prop_columns = prop_factors ? prop_factors + 128 : nullptr;
     a.conj_prop = conj_prop ? 1 : 0; a.out = out;
     enqueue_plane(p, kind, a);
 }
@@ -758,21 +759,17 @@ void enqueue_shift_table_state(cubo_ptycho_plan *p, int st) {
     C2<T> *table = p->shifted.as<C2<T>>() + (size_t)st * p->classes * n;
     timed(p, kShiftTable, 1, [&] { return launch_convert<T>(probe, table, n, s); });
     if (frac == 0) return;
-    if constexpr (std::is_same<T, double>::value) {
-        if (p->plane128) {  // classes 1 .. frac: the probe's spectrum x the class's ramps, inverse FFT, one launch
-            timed(p, kShiftTable, 2, [&] {
-                cudaError_t e = cudaMemcpyAsync(p->spectrum64.ptr, probe, (size_t)n * sizeof(double2),
-                                                cudaMemcpyDeviceToDevice, s);
-                if (e == cudaSuccess) e = launch_fft2_f64(fft64(p), p->spectrum64.as<double2>(), 1, false, s);
-                return e;
-            });
-            Plane128Args a = plane_args(p, kPlaneInverse);
-            a.first = 1; a.count = frac; a.in = p->spectrum64.as<double2>(); a.in_kind = kInputSingle;
-            a.pointwise = kPointwiseFactors; a.prop_rows = p->ramps_r64.as<double2>();
-            a.prop_columns = p->ramps_c64.as<double2>(); a.prop_stride = kSide128; a.out = table;
-            enqueue_plane(p, kShiftTable, a);
-            return;
-        }
+    if (p->fused_shift) {
+        timed(p, kShiftTable, 4, [&] {
+            cudaError_t e = cudaMemcpyAsync(p->spectrum64.ptr, probe, (size_t)n * sizeof(double2),
+                                            cudaMemcpyDeviceToDevice, s);
+            if (e == cudaSuccess) e = launch_fft2_f64(fft64(p), p->spectrum64.as<double2>(), 1, false, s);
+            if (e == cudaSuccess)
+                e = launch_shift_table<T>(fft64(p), p->spectrum64.as<double2>(), p->scratch64.as<double2>(),
+                                          p->ramps_r64.as<double2>(), p->ramps_c64.as<double2>(), frac, table + n, s);
+            return e;
+        });
+        return;
     }
     timed(p, kShiftTable, 2 + 1 + 2 + 1 + 1, [&] {
         cudaError_t e = cudaMemcpyAsync(p->spectrum64.ptr, probe, (size_t)n * sizeof(double2),
@@ -1629,6 +1626,9 @@ int create_plan(cubo_ptycho_context *ctx, const cubo_ptycho_problem *pr, const c
         }
         p->kind_ms.assign(kKinds, 0.0);
         p->kind_launches.assign(kKinds, 0);
+        // the generic variant keeps the line transforms through HBM, for cross-checks
+        p->fused_shift = pp->variant != CUBO_PTYCHO_VARIANT_GENERIC && shift_applicable(p->R, p->C);
+        if (p->fused_shift) check(configure_shift(), "configure shift table");
         p->correct_positions = pp->has_position_correction != 0;  // before the scan tables: one class per position
         if (p->fp64) build_plan<double>(p, pr);
         else build_plan<float>(p, pr);

@@ -229,7 +229,7 @@ __global__ void __cluster_dims__(Q, 1, 1) __launch_bounds__(PlaneGeometry<Q>::kT
     constexpr uint32_t kAmpRowBytes = G::kLines * sizeof(float), kSpanBytes = G::kLines * sizeof(double2);
     // the input and output planes of position p (computed where used: they would hold registers across the kernel)
     auto in_plane = [&]() -> size_t {
-        return (size_t)(a.in_kind == kInputByClass ? a.scan.cls[p] : a.in_kind == kInputSingle ? 0 : p) * kPlane;
+        return (size_t)(a.in_kind == kInputByClass ? a.scan.cls[p] : p) * kPlane;
     };
     auto out_plane = [&]() -> double2 * { return a.out + (size_t)((long long)p * a.out_stride + a.out_offset) * kPlane; };
 
@@ -244,8 +244,7 @@ __global__ void __cluster_dims__(Q, 1, 1) __launch_bounds__(PlaneGeometry<Q>::kT
         const int ii = i >> 4, c = (i >> 3) & 1;
         ti[i] = cconj(a.tw[(ii * (2 * jj + c)) & (kSide - 1)]);
         if (factors) {
-            const size_t off = (size_t)((long long)(p - a.first) * a.prop_stride);
-            double2 r = a.prop_rows[off + i], q = a.prop_columns[off + i];
+            double2 r = a.prop_rows[i], q = a.prop_columns[i];
             if (a.conj_prop) { r.y = -r.y; q.y = -q.y; }
             pr[i] = r;
             pc[i] = q;
