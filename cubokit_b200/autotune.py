@@ -4,10 +4,10 @@ For a problem (detector, object and scan sizes, form) every candidate is timed o
 candidate, a warm-up iteration, then the kernel's device time over a few iterations from the plan's CUDA-event kernel
 statistics.  `tune` picks the object-gather tile (32 x 8, 16 x 16, 64 x 4 pixels, along the residual's contiguous
 axis); `tune_pass` the CTA shape of the shared-memory position pass at the detectors it runs with a compile-time radix
-plan or the FP32 register-line kernel (64 x 64 and 96 x 96).  The fastest candidate is cached in a JSON file keyed by
+plan or the default FP32 kernel (64 x 64 and 96 x 96).  The fastest candidate is cached in a JSON file keyed by
 (what, detector, object, positions, form, GPU name), so the timing runs once per shape per machine.  Neither choice
 changes the object: every object pixel sums the same positions in the same order whatever the tile, and every
-butterfly computes the same values whatever the shared-memory CTA shape; the FP32 register-line kernel agrees with
+butterfly computes the same values whatever the shared-memory CTA shape; the default FP32 kernel agrees with
 those to FP32 round-off.
 """
 from __future__ import annotations

@@ -94,11 +94,11 @@ __device__ __forceinline__ void inner_stage(C2<T> *D, const AnyLine &l, int s, i
 #pragma unroll
         for (int r = 0; r < R; r++) x[r] = x0[r * step];
         if (INV) {
-            twiddle<T, true, R>(x, j, scale, tw);
+            if (sub > 1) twiddle<T, true, R>(x, j, scale, tw);  // blocks of one sample each have none
             regdft::dft<T, true, R>(x);
         } else {
             regdft::dft<T, false, R>(x);
-            twiddle<T, false, R>(x, j, scale, tw);
+            if (sub > 1) twiddle<T, false, R>(x, j, scale, tw);
         }
 #pragma unroll
         for (int r = 0; r < R; r++) x0[r * step] = x[r];
@@ -125,7 +125,7 @@ __device__ __forceinline__ void first_stage(C2<T> *D, const AnyPassArgs<T> &g, i
 #pragma unroll
         for (int r = 0; r < R; r++) x[r] = regdft::turn<C2<T>, false>(x[r], o[r]);
         regdft::dft<T, false, R>(x);
-        twiddle<T, false, R>(x, j, 1, tw);
+        if (sub > 1) twiddle<T, false, R>(x, j, 1, tw);
         C2<T> *y = D + row * g.pitch + j;
 #pragma unroll
         for (int q = 0; q < R; q++) y[q * sub] = x[q];
@@ -144,7 +144,7 @@ __device__ __forceinline__ void last_stage(const C2<T> *D, const AnyPassArgs<T> 
         C2<T> x[R];
 #pragma unroll
         for (int q = 0; q < R; q++) x[q] = y[q * sub];
-        twiddle<T, true, R>(x, j, 1, tw);
+        if (sub > 1) twiddle<T, true, R>(x, j, 1, tw);
         regdft::dft<T, true, R>(x);
         C2<T> *o = out + row * a.columns + j;
 #pragma unroll

@@ -145,14 +145,13 @@ template <typename T> cudaError_t launch_position_pass(const PositionPassArgs<T>
 bool any_pass_applicable(int rows, int columns, bool fp64);
 cudaError_t configure_any_pass();
 template <typename T> cudaError_t launch_any_pass(const PositionPassArgs<T> &a, cudaStream_t s);
-// linepass.cu: the FP32 position pass for 64 x 64 and 96 x 96 detectors with register-resident line transforms (four
-// steps: R-point DFTs in registers, one in-group exchange, G-point DFTs), one CTA per position; the default FP32 pass
-// at those sizes (cubo_ptycho_params.pass_shape 0).
-bool line_pass_applicable(int rows, int columns);
-cudaError_t configure_line_pass();
-cudaError_t launch_line_pass(const PositionPassArgs<float> &a, cudaStream_t s);
-cudaError_t launch_line_pass_grouped(const PositionPassArgs<float> *args, const int *prefix, int items, int total, int N,
-                                     cudaStream_t s);
+// squarepass.cu: the FP32 position pass for 64 x 64 and 96 x 96 detectors, the any-size pass's in-place transforms with
+// the geometry fixed at compile time; the default FP32 pass at those sizes (cubo_ptycho_params.pass_shape 0).
+bool square_pass_applicable(int rows, int columns);
+cudaError_t configure_square_pass();
+cudaError_t launch_square_pass(const PositionPassArgs<float> &a, cudaStream_t s);
+cudaError_t launch_square_pass_grouped(const PositionPassArgs<float> *args, const int *prefix, int items, int total,
+                                       int N, cudaStream_t s);
 
 // Grouped launches (batches of independent reconstructions): every item's units in one persistent launch.  prefix holds
 // items + 1 offsets (item i owns units prefix[i] .. prefix[i + 1] - 1); args one structure per item, in device memory.

@@ -692,7 +692,7 @@ cudaError_t configure_kernels() {
         }
     e = configure_any_pass();
     if (e != cudaSuccess) return e;
-    return configure_line_pass();
+    return configure_square_pass();
 }
 
 size_t position_pass_smem(int n, int rows, int columns, bool fp64) {
@@ -734,7 +734,7 @@ cudaError_t launch_position_pass(const PositionPassArgs<T> &a, int shape, cudaSt
     constexpr int maxn = PassConfig<T>::maxn;
     if (a.count <= 0) return cudaSuccess;
     if constexpr (std::is_same<T, float>::value)
-        if (shape == 0 && line_pass_applicable(a.rows, a.columns)) return launch_line_pass(a, s);
+        if (shape == 0 && square_pass_applicable(a.rows, a.columns)) return launch_square_pass(a, s);
     const size_t smem = pass_smem<T>(a.n, a.rows, a.columns);
     const int threads = a.rows == a.columns ? fixed_threads<T>(a.rows, shape) : 0;
     if (threads > 0)
@@ -755,7 +755,7 @@ cudaError_t launch_position_pass_grouped(const PositionPassArgs<T> *args, const 
                                          int N, int shape, cudaStream_t s) {
     if (total <= 0) return cudaSuccess;
     if constexpr (std::is_same<T, float>::value)
-        if (shape == 0 && line_pass_applicable(N, N)) return launch_line_pass_grouped(args, prefix, items, total, N, s);
+        if (shape == 0 && square_pass_applicable(N, N)) return launch_square_pass_grouped(args, prefix, items, total, N, s);
     const int threads = fixed_threads<T>(N, shape);
     if (threads == 0) return cudaErrorInvalidValue;
     const size_t smem = pass_smem<T>(N * N, N, N);
