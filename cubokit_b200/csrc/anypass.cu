@@ -45,7 +45,7 @@ int any_threads(int rows, int columns) {
 }  // namespace
 
 bool any_pass_applicable(int rows, int columns, bool fp64) {
-    AnyLine r, c;
+    AnyLine r{}, c{};
     if (rows < 2 || columns < 2 || (long long)rows * columns >= 65536 || !plan_line(rows, 31, false, &r) || !plan_line(columns, 31, true, &c)) return false;
     return (fp64 ? any_smem<double>(rows, columns) : any_smem<float>(rows, columns)) <= kAnySmem;
 }

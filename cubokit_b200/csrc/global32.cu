@@ -1,225 +1,292 @@
-// The FP32 position pass for detectors whose plane does not fit one CTA's shared memory (more than 16,384 pixels, sides
-// up to 4096, e.g. 256 x 256), or any detector with CUBO_PTYCHO_VARIANT_GLOBAL.
-//
-// Same arithmetic as the shared-memory pass (exit wave, forward 2-D FFT, Fourier-modulus projection with the 1/n of
-// ifft2 folded in, inverse 2-D FFT; Ptychography.swift:321-350, the Float path PtychographySingle.swift:137-176), in
-// three launches per batch of positions, each reading and writing the residual plane once:
-//
-//  1. rows:    the exit wave X = S O[patch] of nl rows of one position, formed on the way into shared memory, and their
-//              forward row transforms, into dpsi;
-//  2. columns: nl columns of one position: forward column transforms, the projection and its squared residual (one
-//              FP64 partial per CTA, summed over the CTA in a fixed order), inverse column transforms;
-//  3. rows:    the inverse row transforms.
-//
-// The line transforms are the shared-memory Stockham stages of the any-size pass (radices 8/4/2/3/5/7, direct DFT for
-// other primes), nl lines of a CTA at a time; nl is the largest divisor of the line count that keeps nl lines within
-// kG32MaxN elements, so a CTA never straddles two positions and every partial belongs to one position.  Where the
-// lengths keep every address on a 16-byte boundary, the column launch brings its residual columns and amplitudes and
-// the inverse row launch its rows into shared memory by asynchronous 16-byte copies, all in flight at once.  The FP64
-// form has its own global-memory pass (launch_position_pass_global).
-#include "engine.h"
+// Host side of the FP32 position pass through global memory (global32.cuh), its instances with compile-time geometry and
+// the direct DFT.
+#include <algorithm>
+
+#include "global32.cuh"
 
 namespace cubo {
 
 namespace {
 
-constexpr int kG32Threads = 256;
-constexpr int kG32MaxN = 4096;  // complex64 elements of the lines one CTA holds (32 KB)
-// CTAs per SM: 4 for the compile-time plans (64 registers, no spills), 2 for the run-time plan (its per-stage arrays
-// spill at either count)
+// --------------------------------------------------------------------- 128, 192 and 256: geometry at compile time
 
-__device__ __forceinline__ int g32_wrap(int v, int size) { return v < 0 ? v + size : (v >= size ? v - size : v); }
-
-// 16-byte asynchronous copy global -> shared (both addresses 16-byte aligned); completes at g32_copies_wait.
-__device__ __forceinline__ void g32_copy16(uint32_t smem_dst, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void g32_copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-// Waits until at most `pending` of this thread's committed groups are still in flight.
-template <int pending>
-__device__ __forceinline__ void g32_copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(pending) : "memory"); }
-
-// Fixed-order sum over the CTA: warps by shuffles, then thread 0 adds the warp sums in warp order.
-__device__ double g32_block_sum(double v, double *scratch) {
+// Rows of RA RB samples, NL a CTA: RA samples a thread in the outer stage, RB (even, padded by one) in the inner one.
+template <int RA, int RB, int NL, bool INV>
+__global__ void __launch_bounds__(kG32Threads, 4) g32_rows_fixed(const __grid_constant__ G32Args g) {
+    constexpr int L = RA * RB, RL = RB + 1, P = RA * RL;
+    static_assert(RB % 2 == 0, "one pad a block");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const PositionPassArgs<float> &a = g.p;
+    float2 *D = reinterpret_cast<float2 *>(smem_raw);
+    float2 *tw = D + NL * P;
+    const int tid = threadIdx.x;
+    const int p = a.first + (int)(blockIdx.x / g.per), r0 = (int)(blockIdx.x % g.per) * NL;
+    const int rows = min(NL, a.rows - r0);
+    for (int i = tid; i < L; i += kG32Threads) tw[i] = a.tw_columns[i];
+    float2 *io = a.dpsi + (size_t)p * a.n + (size_t)r0 * L;
+    if constexpr (!INV) {
+        const int rr = a.scan.rr[p], cc = a.scan.cc[p], cls = a.scan.cls[p];
+        const float2 *S = a.shifted + (size_t)cls * a.n + (size_t)r0 * L;
+        const bool interior = cc >= L / 2 && cc + L / 2 <= a.object_columns;
+        __syncthreads();
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
-    __syncthreads();
-    double total = 0;
-    if (threadIdx.x == 0)
-        for (int w = 0; w < kG32Threads / 32; w++) total += scratch[w];
-    __syncthreads();
-    return total;  // valid in thread 0
+        for (int i0 = 0; i0 < NL * RB; i0 += kG32Threads) {
+            const int i = i0 + tid, row = i / RB, j = i % RB;
+            if (row < rows) {
+                const float2 *s = S + row * L + j;
+                const float2 *o = a.object + (size_t)g32_wrap(rr + corner_offset(r0 + row, a.rows), a.object_rows) *
+                                             a.object_columns;
+                float2 x[RA], q[RA];
+#pragma unroll
+                for (int r = 0; r < RA; r++) {
+                    const int c = j + r * RB, off = c < L / 2 ? c : c - L;
+                    x[r] = s[r * RB];
+                    q[r] = o[interior ? cc + off : g32_wrap(cc + off, a.object_columns)];
+                }
+#pragma unroll
+                for (int r = 0; r < RA; r++) x[r] = regdft::turn<float2, false>(x[r], q[r]);
+                regdft::dft<float, false, RA>(x);
+                twiddle<float, false, RA>(x, j, 1, tw);
+                float2 *y = D + row * P + j;
+#pragma unroll
+                for (int r = 0; r < RA; r++) y[r * RL] = x[r];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i0 = 0; i0 < NL * RA; i0 += kG32Threads) {
+            const int i = i0 + tid, row = i / RA, K = i % RA;
+            if (row < rows) {
+                const float2 *y = D + row * P + K * RL;
+                float2 x[RB];
+#pragma unroll
+                for (int r = 0; r < RB; r++) x[r] = y[r];
+                regdft::dft<float, false, RB>(x);
+                float2 *o = io + row * L + K;
+#pragma unroll
+                for (int r = 0; r < RB; r++) o[r * RA] = x[r];
+            }
+        }
+    } else {
+#pragma unroll
+        for (int i0 = 0; i0 < NL * RA; i0 += kG32Threads) {
+            const int i = i0 + tid, row = i / RA, K = i % RA;
+            if (row < rows) {
+                const float2 *o = io + row * L + K;
+                float2 x[RB];
+#pragma unroll
+                for (int r = 0; r < RB; r++) x[r] = o[r * RA];
+                regdft::dft<float, true, RB>(x);
+                float2 *y = D + row * P + K * RL;
+#pragma unroll
+                for (int r = 0; r < RB; r++) y[r] = x[r];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i0 = 0; i0 < NL * RB; i0 += kG32Threads) {
+            const int i = i0 + tid, row = i / RB, j = i % RB;
+            if (row < rows) {
+                const float2 *y = D + row * P + j;
+                float2 x[RA];
+#pragma unroll
+                for (int r = 0; r < RA; r++) x[r] = y[r * RL];
+                twiddle<float, true, RA>(x, j, 1, tw);
+                regdft::dft<float, true, RA>(x);
+                float2 *o = io + row * L + j;
+#pragma unroll
+                for (int r = 0; r < RA; r++) o[r * RB] = x[r];
+            }
+        }
+    }
 }
 
-// The line transform of the CTA's lines: the radix plan R0 x R1 x R2 fixed at compile time (R1, R2 = 0: no stage; it
-// must be the plan factor_length gives the line length), or read at run time (R0 = 0).
-template <int R0, int R1, int R2>
-__device__ __forceinline__ void g32_lines_fft(float2 *D, const LineGeom &g, const Radices &rad, const float2 *tw,
-                                              bool inv) {
-    if constexpr (R0 == 0) line_fft<float, kG32Threads, kG32MaxN>(D, g, rad, tw, inv);
-    else line_fft_fixed<float, kG32Threads, kG32MaxN, R0, R1, R2>(D, g, tw, inv);
+// Columns of RA RB samples, NL a CTA: RA samples a thread in the outer stages, RB in the centre step.
+template <int RA, int RB, int NL>
+__global__ void __launch_bounds__(kG32Threads, 4) g32_columns_fixed(const __grid_constant__ G32Args g) {
+    constexpr int L = RA * RB;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ double scratch[kG32Threads / 32];
+    const PositionPassArgs<float> &a = g.p;
+    const int C = a.columns, tid = threadIdx.x;
+    float2 *D = reinterpret_cast<float2 *>(smem_raw);
+    float2 *tw = D + NL * L;
+    const int p = a.first + (int)(blockIdx.x / g.per), c0 = (int)(blockIdx.x % g.per) * NL;
+    const int lines = min(NL, C - c0);
+    float2 *io = a.dpsi + (size_t)p * a.n + c0;
+    const float *A = a.amplitudes + (size_t)p * a.n + c0;
+    for (int i = tid; i < L; i += kG32Threads) {
+        tw[i] = a.tw_rows[i];
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(A + (size_t)i * C));  // the amplitudes, for the centre step
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i0 = 0; i0 < NL * RB; i0 += kG32Threads) {
+        const int i = i0 + tid, j = i / NL, c = i % NL;
+        if (i < NL * RB && c < lines) {
+            const float2 *o = io + (size_t)j * C + c;
+            float2 x[RA];
+#pragma unroll
+            for (int r = 0; r < RA; r++) x[r] = o[(size_t)r * RB * C];
+            regdft::dft<float, false, RA>(x);
+            twiddle<float, false, RA>(x, j, 1, tw);
+            float2 *y = D + j * NL + c;
+#pragma unroll
+            for (int r = 0; r < RA; r++) y[r * RB * NL] = x[r];
+        }
+    }
+    __syncthreads();
+    double err = 0;
+#pragma unroll
+    for (int i0 = 0; i0 < NL * RA; i0 += kG32Threads) {
+        const int i = i0 + tid, b = i / NL, c = i % NL;
+        if (i < NL * RA && c < lines) {
+            const float *am = A + (size_t)b * C + c;  // output q of block b is the frequency b + RA q
+            float measured[RB];
+#pragma unroll
+            for (int q = 0; q < RB; q++) measured[q] = am[(size_t)q * RA * C];
+            float2 *y = D + b * RB * NL + c;
+            float2 x[RB];
+#pragma unroll
+            for (int r = 0; r < RB; r++) x[r] = y[r * NL];
+            regdft::dft<float, false, RB>(x);
+#pragma unroll
+            for (int q = 0; q < RB; q++) x[q] = g32_project(x[q], measured[q], a.inv_n, err);
+            regdft::dft<float, true, RB>(x);
+#pragma unroll
+            for (int r = 0; r < RB; r++) y[r * NL] = x[r];
+        }
+    }
+    const double total = g32_block_sum(err, scratch);  // its barriers also order the centre step before the inverse one
+    if (tid == 0) a.error[(size_t)p * g.per + c0 / NL] = total;
+#pragma unroll
+    for (int i0 = 0; i0 < NL * RB; i0 += kG32Threads) {
+        const int i = i0 + tid, j = i / NL, c = i % NL;
+        if (i < NL * RB && c < lines) {
+            const float2 *y = D + j * NL + c;
+            float2 x[RA];
+#pragma unroll
+            for (int r = 0; r < RA; r++) x[r] = y[r * RB * NL];
+            twiddle<float, true, RA>(x, j, 1, tw);
+            regdft::dft<float, true, RA>(x);
+            float2 *o = io + (size_t)j * C + c;
+#pragma unroll
+            for (int r = 0; r < RA; r++) o[(size_t)r * RB * C] = x[r];
+        }
+    }
 }
 
-// Rows r0 .. r0 + nl - 1 of position p = first + block / (rows / nl): with exit_wave the rows of X = S O[patch] (the
-// window corner-centred and periodic in the object), else the rows dpsi holds; transformed along the row (forward, or
-// inverse with inv) and written to dpsi.
-// NL > 0 (compile-time plans only): nl == NL and the line length is R0 R1 R2, so the line geometry is a compile-time
-// constant and the transform's index arithmetic folds.
-template <int R0, int R1, int R2, int NL>
-__global__ void __launch_bounds__(kG32Threads, R0 ? 4 : 2)
-    g32_rows_kernel(PositionPassArgs<float> a, int nl_arg, int exit_wave, int inv) {
+// ---------------------------------------------------------------- direct DFT, lengths with a prime factor above 31
+
+// nl rows of one position: the exit wave's (exit_wave) or dpsi's, transformed forward or (inv) back into dpsi.
+__global__ void __launch_bounds__(kG32Threads, 2)
+    g32_rows_direct(PositionPassArgs<float> a, int nl, int exit_wave, int inv) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2 *D = reinterpret_cast<float2 *>(smem_raw);
-    const int L = NL ? R0 * (R1 ? R1 : 1) * (R2 ? R2 : 1) : a.columns;
-    const int nl = NL ? NL : nl_arg;
+    const int L = a.columns;
     float2 *tw = D + (size_t)nl * L;
     for (int i = threadIdx.x; i < L; i += kG32Threads) tw[i] = a.tw_columns[i];
     const int per = a.rows / nl;
     const int p = a.first + (int)(blockIdx.x / per), r0 = (int)(blockIdx.x % per) * nl;
     float2 *rows = a.dpsi + (size_t)p * a.n + (size_t)r0 * L;
-    if (exit_wave) {
-        const int rr = a.scan.rr[p], cc = a.scan.cc[p], cls = a.scan.cls[p];
-        const float2 *S = a.shifted + (size_t)cls * a.n + (size_t)r0 * L;
-        for (int i = threadIdx.x; i < nl * L; i += kG32Threads) {
-            const int j = i / L, e = i - j * L;
-            const int y = g32_wrap(rr + corner_offset(r0 + j, a.rows), a.object_rows);
-            const int x = g32_wrap(cc + corner_offset(e, a.columns), a.object_columns);
-            D[i] = cmul(S[i], a.object[(size_t)y * a.object_columns + x]);
-        }
-    } else if ((L & 1) == 0) {  // the rows are contiguous and start on a 16-byte boundary: every copy in flight at once
-        const uint32_t d0 = (uint32_t)__cvta_generic_to_shared(D);
-        for (int i = threadIdx.x; i < nl * L / 2; i += kG32Threads) g32_copy16(d0 + 16u * (uint32_t)i, rows + 2 * i);
-        g32_copies_commit();
-        g32_copies_wait<0>();
-    } else {
-        for (int i = threadIdx.x; i < nl * L; i += kG32Threads) D[i] = rows[i];
+    const int rr = a.scan.rr[p], cc = a.scan.cc[p], cls = a.scan.cls[p];
+    const float2 *S = a.shifted + (size_t)cls * a.n + (size_t)r0 * L;
+    for (int i = threadIdx.x; i < nl * L; i += kG32Threads) {
+        if (!exit_wave) { D[i] = rows[i]; continue; }
+        const int j = i / L, e = i - j * L;
+        const int y = g32_wrap(rr + corner_offset(r0 + j, a.rows), a.object_rows);
+        const int x = g32_wrap(cc + corner_offset(e, a.columns), a.object_columns);
+        D[i] = cmul(S[i], a.object[(size_t)y * a.object_columns + x]);
     }
     __syncthreads();
-    g32_lines_fft<R0, R1, R2>(D, LineGeom{L, nl, 1, L}, a.rad_columns, tw, inv != 0);
+    direct_lines<float, kG32Threads, kG32MaxN / kG32Threads>(D, LineGeom{L, nl, 1, L}, tw, inv != 0);
     for (int i = threadIdx.x; i < nl * L; i += kG32Threads) rows[i] = D[i];
 }
 
-// Columns c0 .. c0 + nl - 1 of position p = first + block / (columns / nl), staged with element e of column j at
-// D[e nl + j] (consecutive threads read consecutive columns of one row): forward column transforms, the Fourier-modulus
-// projection (Ptychography.swift:338-349) with the inverse's 1/n folded in and its squared residual, inverse column
-// transforms.  The residual of the CTA's pixels goes to error[p (columns / nl) + c0 / nl].
-template <int R0, int R1, int R2, int NL>
-__global__ void __launch_bounds__(kG32Threads, R0 ? 4 : 2) g32_columns_kernel(PositionPassArgs<float> a, int nl_arg) {
+// nl columns of one position, element e of column j at D[e nl + j].
+__global__ void __launch_bounds__(kG32Threads, 2) g32_columns_direct(PositionPassArgs<float> a, int nl) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ double scratch[kG32Threads / 32];
     float2 *D = reinterpret_cast<float2 *>(smem_raw);
-    const int L = NL ? R0 * (R1 ? R1 : 1) * (R2 ? R2 : 1) : a.rows;
-    const int nl = NL ? NL : nl_arg;
+    const int L = a.rows;
     float2 *tw = D + (size_t)nl * L;
-    float *As = reinterpret_cast<float *>(tw + L);  // the CTA's amplitudes, staged like D
     for (int i = threadIdx.x; i < L; i += kG32Threads) tw[i] = a.tw_rows[i];
     const int per = a.columns / nl;
     const int p = a.first + (int)(blockIdx.x / per), c0 = (int)(blockIdx.x % per) * nl;
     float2 *base = a.dpsi + (size_t)p * a.n + c0;
     const float *A = a.amplitudes + (size_t)p * a.n + c0;
-    // nl and the row length multiples of 4 and the column length even (so every copy's source and destination, the
-    // amplitude area As included, start on 16-byte boundaries): the residual columns in pairs and the amplitudes in
-    // fours by asynchronous copies, every copy in flight at once; the amplitudes land while the forward transforms run
-    const bool staged = (nl & 3) == 0 && (a.columns & 3) == 0 && (L & 1) == 0;
-    if (staged) {
-        const uint32_t d0 = (uint32_t)__cvta_generic_to_shared(D), a0 = (uint32_t)__cvta_generic_to_shared(As);
-        const int pairs = nl / 2, quads = nl / 4;
-        for (int i = threadIdx.x; i < pairs * L; i += kG32Threads) {
-            const int e = i / pairs, j = 2 * (i - e * pairs);
-            g32_copy16(d0 + 8u * (uint32_t)(e * nl + j), base + (size_t)e * a.columns + j);
-        }
-        g32_copies_commit();
-        for (int i = threadIdx.x; i < quads * L; i += kG32Threads) {
-            const int e = i / quads, j = 4 * (i - e * quads);
-            g32_copy16(a0 + 4u * (uint32_t)(e * nl + j), A + (size_t)e * a.columns + j);
-        }
-        g32_copies_commit();
-        g32_copies_wait<1>();  // the residual columns; the amplitudes may still be in flight
-    } else {
-        for (int i = threadIdx.x; i < nl * L; i += kG32Threads) {
-            const int e = i / nl, j = i - e * nl;
-            D[i] = base[(size_t)e * a.columns + j];
-            As[i] = A[(size_t)e * a.columns + j];
-        }
+    for (int i = threadIdx.x; i < nl * L; i += kG32Threads) {
+        const int e = i / nl, j = i - e * nl;
+        D[i] = base[(size_t)e * a.columns + j];
     }
     __syncthreads();
     const LineGeom geom{L, nl, nl, 1};
-    g32_lines_fft<R0, R1, R2>(D, geom, a.rad_rows, tw, false);
-    if (staged) {
-        g32_copies_wait<0>();
-        __syncthreads();
-    }
+    direct_lines<float, kG32Threads, kG32MaxN / kG32Threads>(D, geom, tw, false);
     double err = 0;
     for (int i = threadIdx.x; i < nl * L; i += kG32Threads) {
-        const float2 f = D[i];
-        const float mag = sqrtf(f.x * f.x + f.y * f.y);
-        const float measured = As[i];
-        const float miss = measured - mag;
-        err += (double)(miss * miss);
-        if (mag > 0.f) {
-            const float s = (measured / mag - 1.f) * a.inv_n;
-            D[i] = make_float2(f.x * s, f.y * s);
-        } else {
-            D[i] = make_float2(measured * a.inv_n, 0.f);
-        }
+        const int e = i / nl, j = i - e * nl;
+        D[i] = g32_project(D[i], A[(size_t)e * a.columns + j], a.inv_n, err);
     }
     const double total = g32_block_sum(err, scratch);  // its barriers also order the projection before the inverse
     if (threadIdx.x == 0) a.error[(size_t)p * per + c0 / nl] = total;
-    g32_lines_fft<R0, R1, R2>(D, geom, a.rad_rows, tw, true);
+    direct_lines<float, kG32Threads, kG32MaxN / kG32Threads>(D, geom, tw, true);
     for (int i = threadIdx.x; i < nl * L; i += kG32Threads) {
         const int e = i / nl, j = i - e * nl;
         base[(size_t)e * a.columns + j] = D[i];
     }
 }
 
-// The largest divisor d of `lines` with d line_length <= kG32MaxN: lines per CTA.
-int g32_lines(int line_length, int lines) {
+// -------------------------------------------------------------------------------------------------------- host side
+
+// Direct: the largest divisor d of `lines` with d line_length <= kG32MaxN.
+int g32_divisor_lines(int line_length, int lines) {
     int best = 1;
     for (int d = 1; d <= lines && (long long)d * line_length <= kG32MaxN; d++)
         if (lines % d == 0) best = d;
     return best;
 }
 
-// Dynamic shared memory: nl lines and the twiddle table (complex64), and for the columns launch the amplitudes (Float32).
-size_t g32_smem(int nl, int line_length, bool amplitudes) {
-    return ((size_t)nl * line_length + line_length) * sizeof(float2) +
-           (amplitudes ? (size_t)nl * line_length * sizeof(float) : 0);
+// Lines per CTA of the planned launches: the power of two that fills kG32MaxN elements; for columns at least 16 (whole
+// 128-byte segments of each row) while those fit a third of the SM.  The last CTA of a position may hold fewer.
+int g32_lines(int line_length, bool columns) {
+    int nl = 1;
+    while (2 * nl * line_length <= kG32MaxN) nl *= 2;
+    if (columns)
+        while (nl < 16 && 2 * nl * line_length * sizeof(float2) <= 72 * 1024) nl *= 2;
+    return nl;
 }
 
-using RowsKernel = void (*)(PositionPassArgs<float>, int, int, int);
-using ColumnsKernel = void (*)(PositionPassArgs<float>, int);
+struct G32Plan {
+    AnyLine line{};
+    bool planned = false;  // else the direct DFT
+    int nl = 1;
+    size_t smem = 0;
+    G32Kernel forward = nullptr, inverse = nullptr, columns = nullptr;
+};
 
-// Which compile-time plan `rad` is: 1..4 for lines of 128 (8 8 2), 192 (8 8 3), 256 (8 8 4), 512 (8 8 8), else 0 (the
-// run-time plan).
-int g32_plan_index(const Radices &rad) {
-    auto is = [&](int a, int b, int c) {
-        const int want[3] = {a, b, c};
-        if (rad.count != 3) return false;
-        for (int i = 0; i < 3; i++)
-            if (rad.r[i] != want[i]) return false;
-        return true;
-    };
-    return is(8, 8, 2) ? 1 : is(8, 8, 3) ? 2 : is(8, 8, 4) ? 3 : is(8, 8, 8) ? 4 : 0;
-}
-// The lines per CTA of each plan's folded instance (the largest power of two within kG32MaxN elements).
-constexpr int kFoldLines[5] = {0, 32, 16, 16, 8};
-RowsKernel rows_instance(int i, bool folded) {
-    constexpr RowsKernel k[5] = {g32_rows_kernel<0, 0, 0, 0>, g32_rows_kernel<8, 8, 2, 0>, g32_rows_kernel<8, 8, 3, 0>,
-                                 g32_rows_kernel<8, 8, 4, 0>, g32_rows_kernel<8, 8, 8, 0>};
-    constexpr RowsKernel f[5] = {g32_rows_kernel<0, 0, 0, 0>, g32_rows_kernel<8, 8, 2, 32>,
-                                 g32_rows_kernel<8, 8, 3, 16>, g32_rows_kernel<8, 8, 4, 16>,
-                                 g32_rows_kernel<8, 8, 8, 8>};
-    return folded ? f[i] : k[i];
-}
-ColumnsKernel columns_instance(int i, bool folded) {
-    constexpr ColumnsKernel k[5] = {g32_columns_kernel<0, 0, 0, 0>, g32_columns_kernel<8, 8, 2, 0>,
-                                    g32_columns_kernel<8, 8, 3, 0>, g32_columns_kernel<8, 8, 4, 0>,
-                                    g32_columns_kernel<8, 8, 8, 0>};
-    constexpr ColumnsKernel f[5] = {g32_columns_kernel<0, 0, 0, 0>, g32_columns_kernel<8, 8, 2, 32>,
-                                    g32_columns_kernel<8, 8, 3, 16>, g32_columns_kernel<8, 8, 4, 16>,
-                                    g32_columns_kernel<8, 8, 8, 8>};
-    return folded ? f[i] : k[i];
+G32Plan g32_plan(int L, bool columns) {
+    G32Plan p;
+    p.planned = L >= 2 && plan_line(L, 31, !columns, &p.line);
+    if (!p.planned) return p;
+    p.nl = g32_lines(L, columns);
+    bool w = false;
+    for (int i = 0; i < p.line.stages; i++) w = w || p.line.r[i] > 16;
+    const size_t last = (size_t)p.line.r[p.line.stages - 1];
+    p.smem = columns ? ((size_t)p.nl * L + L) * sizeof(float2) + L * sizeof(unsigned short)
+                     : ((size_t)p.nl * (L / last) * (last | 1) + L) * sizeof(float2) + L * sizeof(unsigned short);
+    if (columns) {
+        p.columns = w ? g32_wide_columns() : g32_columns<false>;
+        if (L == 128) p.columns = g32_columns_fixed<16, 8, 32>;
+        if (L == 192) p.columns = g32_columns_fixed<16, 12, 16>;
+        if (L == 256) p.columns = g32_columns_fixed<16, 16, 16>;
+    } else {
+        p.forward = w ? g32_wide_rows_forward() : g32_rows_forward<false>;
+        p.inverse = w ? g32_wide_rows_inverse() : g32_rows_inverse<false>;
+        if (L == 128) { p.forward = g32_rows_fixed<8, 16, 32, false>; p.inverse = g32_rows_fixed<8, 16, 32, true>; }
+        if (L == 192) { p.forward = g32_rows_fixed<12, 16, 16, false>; p.inverse = g32_rows_fixed<12, 16, 16, true>; }
+        if (L == 256) { p.forward = g32_rows_fixed<16, 16, 16, false>; p.inverse = g32_rows_fixed<16, 16, 16, true>; }
+    }
+    return p;
 }
 
 }  // namespace
@@ -228,48 +295,71 @@ bool global32_applicable(int rows, int columns) {
     return rows >= 1 && columns >= 1 && rows <= kG32MaxN && columns <= kG32MaxN;
 }
 
-int global32_partials_per_position(int rows, int columns) { return columns / g32_lines(rows, columns); }
+int global32_partials_per_position(int rows, int columns) {
+    const G32Plan p = g32_plan(rows, true);
+    return p.planned ? (columns + p.nl - 1) / p.nl : columns / g32_divisor_lines(rows, columns);
+}
 
 cudaError_t configure_global32() {
-    // at most kG32MaxN elements and their amplitudes, a twiddle table of at most kG32MaxN
-    const int bytes = (int)((kG32MaxN + kG32MaxN) * sizeof(float2) + kG32MaxN * sizeof(float));
-    for (int i = 0; i < 5; i++)
-        for (bool folded : {false, true}) {
-            cudaError_t e = cudaFuncSetAttribute(rows_instance(i, folded), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 bytes);
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(columns_instance(i, folded), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         bytes);
-            if (e != cudaSuccess) return e;
-        }
-    return cudaSuccess;
+    const G32Kernel kernels[] = {g32_rows_forward<false>, g32_rows_inverse<false>, g32_columns<false>,
+                                 g32_wide_rows_forward(), g32_wide_rows_inverse(), g32_wide_columns(),
+                                 g32_columns_fixed<16, 8, 32>, g32_columns_fixed<16, 12, 16>,
+                                 g32_columns_fixed<16, 16, 16>, g32_rows_fixed<8, 16, 32, false>,
+                                 g32_rows_fixed<8, 16, 32, true>, g32_rows_fixed<12, 16, 16, false>,
+                                 g32_rows_fixed<12, 16, 16, true>, g32_rows_fixed<16, 16, 16, false>,
+                                 g32_rows_fixed<16, 16, 16, true>};
+    for (G32Kernel k : kernels) {
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kG32Smem);
+        if (e != cudaSuccess) return e;
+    }
+    cudaError_t e = cudaFuncSetAttribute(g32_rows_direct, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kG32Smem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(g32_columns_direct, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kG32Smem);
+    return e;
 }
 
 cudaError_t launch_position_pass_global32(const PositionPassArgs<float> &a, int *launches, cudaStream_t s) {
     if (launches) *launches = 0;
     if (a.count <= 0) return cudaSuccess;
     if (!global32_applicable(a.rows, a.columns)) return cudaErrorInvalidValue;
-    const int nr = g32_lines(a.columns, a.rows), nc = g32_lines(a.rows, a.columns);
-    const int per_r = a.rows / nr, per_c = a.columns / nc;
-    const size_t smem_r = g32_smem(nr, a.columns, false), smem_c = g32_smem(nc, a.rows, true);
-    const int ir = g32_plan_index(a.rad_columns), ic = g32_plan_index(a.rad_rows);  // row lines: length columns
-    const RowsKernel rows_k = rows_instance(ir, ir > 0 && nr == kFoldLines[ir]);
-    const ColumnsKernel columns_k = columns_instance(ic, ic > 0 && nc == kFoldLines[ic]);
-    // batches of positions whose CTAs fit one grid dimension
+    const G32Plan pr = g32_plan(a.columns, false), pc = g32_plan(a.rows, true);
+    const int nr = pr.planned ? pr.nl : g32_divisor_lines(a.columns, a.rows);
+    const int nc = pc.planned ? pc.nl : g32_divisor_lines(a.rows, a.columns);
+    const int per_r = (a.rows + nr - 1) / nr, per_c = (a.columns + nc - 1) / nc;
+    const size_t direct_r = ((size_t)nr + 1) * a.columns * sizeof(float2);
+    const size_t direct_c = ((size_t)nc + 1) * a.rows * sizeof(float2);
+    auto args = [](const G32Plan &p, int per) {
+        G32Args g{};
+        g.line = p.line;
+        g.nl = p.nl;
+        g.per = per;
+        g.by_nl = divisor(p.nl);
+        for (int i = 0; i < p.line.stages; i++) g.by_block[i] = divisor(p.line.L / p.line.r[i]);
+        return g;
+    };
+    G32Args gr = args(pr, per_r), gc = args(pc, per_c);
+    // Batches of positions whose CTAs fit one grid dimension.  (Batches small enough to stay in L2 between their launches,
+    // 19 to 111 MB of residuals, measured slower: 2.95 to 4.29 ms against 2.51 at 4,096 positions of 256 x 256; the gaps and
+    // part waves of 3 launches a batch cost more than the HBM traffic they save.)
     const int chunk = (int)std::max<long long>(1, (1LL << 30) / std::max(per_r, per_c));
     int count = 0;
     for (int first = 0; first < a.count; first += chunk) {
         PositionPassArgs<float> b = a;
         b.first = a.first + first;
+        gr.p = gc.p = b;
         const int m = std::min(chunk, a.count - first);
-        rows_k<<<(unsigned)((long long)m * per_r), kG32Threads, smem_r, s>>>(b, nr, 1, 0);
+        const unsigned grid_r = (unsigned)((long long)m * per_r), grid_c = (unsigned)((long long)m * per_c);
+        if (pr.planned) pr.forward<<<grid_r, kG32Threads, pr.smem, s>>>(gr);
+        else g32_rows_direct<<<grid_r, kG32Threads, direct_r, s>>>(b, nr, 1, 0);
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) {
-            columns_k<<<(unsigned)((long long)m * per_c), kG32Threads, smem_c, s>>>(b, nc);
+            if (pc.planned) pc.columns<<<grid_c, kG32Threads, pc.smem, s>>>(gc);
+            else g32_columns_direct<<<grid_c, kG32Threads, direct_c, s>>>(b, nc);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) {
-            rows_k<<<(unsigned)((long long)m * per_r), kG32Threads, smem_r, s>>>(b, nr, 0, 1);
+            if (pr.planned) pr.inverse<<<grid_r, kG32Threads, pr.smem, s>>>(gr);
+            else g32_rows_direct<<<grid_r, kG32Threads, direct_r, s>>>(b, nr, 0, 1);
             e = cudaGetLastError();
         }
         if (e != cudaSuccess) return e;

@@ -159,7 +159,7 @@ int shift_fold(int rows, int columns, AnyLine *lines, AnyLine *columns_line) {
 }  // namespace
 
 bool shift_applicable(int rows, int columns) {
-    AnyLine l, c;
+    AnyLine l{}, c{};
     return shift_fold(rows, columns, &l, &c) > 0;
 }
 
