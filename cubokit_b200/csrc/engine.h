@@ -35,18 +35,23 @@ struct ObjectGatherArgs {
     int rows, columns, object_rows, object_columns, n;
     int tiles_x;               // tiles per object row
     int tile_w, tile_h;        // tile shape, tile_w x tile_h = kGatherThreads pixels
-    const int *tile_start;     // CSR offsets, [tiles + 1]
-    const int *tile_list;      // position indices, ascending within each tile
+    const int *tile_start;     // CSR offsets, [tiles * groups + 1]
+    const int *tile_list;      // position indices, ascending within each tile's group
     ScanTables scan;
     const C2<T> *shifted;
     const C2<T> *dpsi;
     C2<T> *grad;               // object gradient sum conj(S) dpsi
     T *weight;                 // sum |S|^2
-    double *tile_max;          // per-tile max of weight
+    double *tile_max;          // max of weight, per tile (one group) or per 256 pixels (object_combine_blocks)
+    // each tile's candidates in `groups` shares (object_gather_groups), each summed by a CTA of its own into
+    // part_grad / part_weight [group][pixel], then added in order
+    int groups = 1;
+    C2<T> *part_grad = nullptr;
+    T *part_weight = nullptr;
     int states = 1;            // mixed state (FP64): dpsi and shifted hold one block per state, these strides apart
     long long dpsi_state_stride = 0, shifted_state_stride = 0;
-    // One band of the positions ([band_first, band_end), single state): block b takes tile band_tiles[b] and only its
-    // candidates inside the band, whose residuals dpsi holds from position band_first on.  A tile's sums start from
+    // One band of the positions ([band_first, band_end), single state): block b takes part band_tiles[b] (tile x groups +
+    // group) and only its candidates inside the band, whose residuals dpsi holds from position band_first on.  A tile's sums start from
     // the values grad / weight hold unless the band holds its first candidate, and its tile_max is written by the
     // band that holds its last one (or by the band that lists it with no candidates at all).  nullptr: every tile,
     // every candidate, dpsi from position 0.
@@ -162,9 +167,15 @@ template <typename T> cudaError_t launch_position_pass_grouped(const PositionPas
                                                                int items, int total, int N, int shape, cudaStream_t s);
 template <typename T> cudaError_t launch_object_gather_grouped(const ObjectGatherArgs<T> *args, const int *prefix,
                                                                int items, int total, cudaStream_t s);
+template <typename T> cudaError_t launch_object_combine_grouped(const ObjectGatherArgs<T> *args, const int *prefix,
+                                                                int items, int total, cudaStream_t s);
 template <typename T> cudaError_t launch_probe_gather_grouped(const ProbeGatherArgs<T> *args, const int *prefix,
                                                               int items, int total, cudaStream_t s);
-template <typename T> cudaError_t launch_object_gather(const ObjectGatherArgs<T> &a, int tiles, cudaStream_t s);
+int object_gather_groups(long long objects, int positions);  // shares of each tile's candidates
+int object_combine_blocks(int object_rows, int object_columns);
+// the gather over `parts` tiles x groups (or a band's list of them), and with several groups the sum of their partials
+template <typename T> cudaError_t launch_object_combine(const ObjectGatherArgs<T> &a, cudaStream_t s);
+template <typename T> cudaError_t launch_object_gather(const ObjectGatherArgs<T> &a, int parts, cudaStream_t s);
 template <typename T> cudaError_t launch_probe_gather(const ProbeGatherArgs<T> &a, cudaStream_t s);
 template <typename T> int probe_gather_resident_ctas();  // CTAs of the probe gather resident on one SM (at least 1)
 template <typename T>
@@ -180,8 +191,9 @@ cudaError_t launch_object_update(C2<T> *object, const C2<T> *grad, const T *weig
 cudaError_t launch_error_reduce(const double *error, long long count, double divisor, double *errors, int *iteration,
                                 double *scratch, cudaStream_t s);
 int error_reduce_scratch();  // doubles of scratch launch_error_reduce needs
-// object-gather candidate lists on the device: without `list`, counts[tile] = the number of positions whose window
-// touches the tile; with it (and starts = exclusive sums of the counts), those positions in ascending order
+// object-gather candidate lists on the device: without `list`, counts[tile * groups + group] = the number of the group's
+// positions whose window touches the tile; with it (and starts = exclusive sums of the counts), those positions in
+// ascending order
 template <typename T>
 cudaError_t launch_object_cap(C2<T> *object, int count, int pure_phase, cudaStream_t s);
 
@@ -208,8 +220,8 @@ cudaError_t launch_exclusive_scan(const int *counts, int tiles, int *starts, lon
 cudaError_t launch_position_center(double *positions, int count, double initial_mean_row, double initial_mean_column,
                                    cudaStream_t s);
 cudaError_t launch_tile_lists(const int *rr, const int *cc, int count, int rows, int columns, int object_rows,
-                              int object_columns, int tile_w, int tile_h, int tiles_x, int tiles, int *counts,
-                              const int *starts, int *list, int capacity, cudaStream_t s);
+                              int object_columns, int tile_w, int tile_h, int tiles_x, int tiles, int groups,
+                              int *counts, const int *starts, int *list, int capacity, cudaStream_t s);
 // sum A^2 of `count` amplitudes into scratch[amplitude_check_scratch() - 1] (FP64, fixed order); *bad = 1 if any is not
 // finite and non-negative (*bad is not cleared)
 cudaError_t launch_amplitude_check(const float *amplitudes, long long count, double *scratch, int *bad, cudaStream_t s);

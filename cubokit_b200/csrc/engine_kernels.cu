@@ -224,7 +224,8 @@ __device__ __forceinline__ void object_gather_body(const ObjectGatherArgs<T> &a,
     __shared__ int s_p[kGatherChunk], s_cls[kGatherChunk];
     __shared__ int s_off[kGatherChunk][kMaxTileSide + kGatherThreads / kMaxTileSide + 4];  // rows, then columns
     __shared__ double scratch[32];
-    const int tile = a.band_tiles ? a.band_tiles[unit] : unit;
+    const int part = a.band_tiles ? a.band_tiles[unit] : unit;  // one group of a tile's candidates
+    const int tile = part / a.groups, group = part - tile * a.groups;
     const int tx = tile % a.tiles_x, ty = tile / a.tiles_x;
     const int x0 = tx * a.tile_w, y0 = ty * a.tile_h;
     // consecutive threads take consecutive object columns, hence consecutive addresses of each [row][column] residual
@@ -234,15 +235,18 @@ __device__ __forceinline__ void object_gather_body(const ObjectGatherArgs<T> &a,
     constexpr int kInvalid = -(1 << 30);
     C2<T> g = mk<T>(0, 0);
     T w = 0;
-    const int list_begin = a.tile_start[tile], list_end = a.tile_start[tile + 1];
+    // where this group's sums go: with several groups into its share of the partials, which object_combine_kernel adds
+    C2<T> *sum_grad = a.groups > 1 ? a.part_grad : a.grad;
+    T *sum_weight = a.groups > 1 ? a.part_weight : a.weight;
+    const size_t j = ((size_t)group * a.object_rows + y) * a.object_columns + x;
+    const int list_begin = a.tile_start[part], list_end = a.tile_start[part + 1];
     int begin = list_begin, end = list_end;
     if (a.band_tiles) {  // this band's candidates only; the running sums continue from memory after the first band
         begin = lower_bound_index(a.tile_list, list_begin, list_end, a.band_first);
         end = lower_bound_index(a.tile_list, begin, list_end, a.band_end);
         if (begin != list_begin && inside) {
-            const size_t j = (size_t)y * a.object_columns + x;
-            g = a.grad[j];
-            w = a.weight[j];
+            g = sum_grad[j];
+            w = sum_weight[j];
         }
     }
     for (int base = begin; base < end; base += kGatherChunk) {
@@ -327,11 +331,10 @@ __device__ __forceinline__ void object_gather_body(const ObjectGatherArgs<T> &a,
         }
     }
     if (inside) {
-        const size_t j = (size_t)y * a.object_columns + x;
-        a.grad[j] = g;
-        a.weight[j] = w;
+        sum_grad[j] = g;
+        sum_weight[j] = w;
     }
-    if (end != list_end) return;  // a later band still adds to this tile (uniform over the block)
+    if (end != list_end || a.groups > 1) return;  // a later band or another group still adds (uniform over the block)
     const double m = block_max<kGatherThreads>(inside ? (double)w : -DBL_MAX, scratch);
     if (threadIdx.x == 0) a.tile_max[tile] = m;
 }
@@ -341,7 +344,31 @@ __global__ void __launch_bounds__(kGatherThreads) object_gather_kernel(ObjectGat
     object_gather_body<T, MIXED>(a, blockIdx.x);
 }
 
-// Grouped object gather: the tiles of every item in one launch, one CTA per (item, tile) unit.
+// The groups' object sums added in order, and each block's maximum of the weights.
+template <typename T>
+__device__ __forceinline__ void object_combine_body(const ObjectGatherArgs<T> &a, int block) {
+    __shared__ double scratch[32];
+    const long long objects = (long long)a.object_rows * a.object_columns, j = (long long)block * kGatherThreads + threadIdx.x;
+    C2<T> g = mk<T>(0, 0);
+    T w = 0;
+    if (j < objects) {
+        for (int k = 0; k < a.groups; k++) {
+            g = cadd(g, a.part_grad[k * objects + j]);
+            w += a.part_weight[k * objects + j];
+        }
+        a.grad[j] = g;
+        a.weight[j] = w;
+    }
+    const double m = block_max<kGatherThreads>(j < objects ? (double)w : -DBL_MAX, scratch);
+    if (threadIdx.x == 0) a.tile_max[block] = m;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kGatherThreads) object_combine_kernel(ObjectGatherArgs<T> a) {
+    object_combine_body<T>(a, blockIdx.x);
+}
+
+// Grouped object gather: the tiles of every item in one launch, one CTA per (item, tile and group) unit.
 template <typename T>
 __global__ void __launch_bounds__(kGatherThreads) object_gather_grouped_kernel(const ObjectGatherArgs<T> *args,
                                                                                const int *prefix, int items, int total) {
@@ -349,6 +376,16 @@ __global__ void __launch_bounds__(kGatherThreads) object_gather_grouped_kernel(c
     const int it = group_item(prefix, items, u);
     const ObjectGatherArgs<T> a = args[it];
     object_gather_body<T, false>(a, u - prefix[it]);
+}
+
+// Grouped combine: every item's blocks of 256 object pixels, one CTA per unit.
+template <typename T>
+__global__ void __launch_bounds__(kGatherThreads) object_combine_grouped_kernel(const ObjectGatherArgs<T> *args,
+                                                                                const int *prefix, int items, int total) {
+    const int u = blockIdx.x;
+    const int it = group_item(prefix, items, u);
+    const ObjectGatherArgs<T> a = args[it];
+    object_combine_body<T>(a, u - prefix[it]);
 }
 
 // ------------------------------------------------------------------------------------------------ candidate lists
@@ -360,21 +397,23 @@ __device__ __forceinline__ bool cyclic_overlap(int start, int length, int t0, in
     return d < length || d + len > size;
 }
 
-// One warp per object-gather tile: the positions whose window touches the tile, in ascending order.  Without `list`
-// it counts them into counts[tile]; with it, it writes them from starts[tile] on.  A window covers the object rows
+// One warp per part (one of `groups` shares of an object-gather tile: the runs of 32 positions whose index is the group's
+// modulo groups): the positions whose window touches the tile, in ascending order.  Without `list` it counts them into
+// counts[part]; with it, it writes them from starts[part] on.  A window covers the object rows
 // rr - rows/2 .. rr + (rows+1)/2 - 1 and the columns likewise, wrapped.
 __global__ void __launch_bounds__(256) tile_lists_kernel(const int *rr, const int *cc, int count, int rows, int columns,
                                                          int object_rows, int object_columns, int tile_w, int tile_h,
-                                                         int tiles_x, int tiles, int *counts, const int *starts,
-                                                         int *list, int capacity) {
-    const int tile = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (tile >= tiles) return;
+                                                         int tiles_x, int tiles, int groups, int *counts,
+                                                         const int *starts, int *list, int capacity) {
+    const int part = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (part >= tiles * groups) return;
+    const int tile = part / groups, group = part - tile * groups;
     const int ty = tile / tiles_x, tx = tile - ty * tiles_x;
     const int y0 = ty * tile_h, x0 = tx * tile_w;
     const int hy = min(tile_h, object_rows - y0), hx = min(tile_w, object_columns - x0);
     int n = 0;
-    const int base = list ? starts[tile] : 0;
-    for (int i0 = 0; i0 < count; i0 += 32) {
+    const int base = list ? starts[part] : 0;
+    for (int i0 = 32 * group; i0 < count; i0 += 32 * groups) {
         const int i = i0 + lane;
         const bool hit = i < count && cyclic_overlap(rr[i] - rows / 2, rows, y0, hy, object_rows) &&
                          cyclic_overlap(cc[i] - columns / 2, columns, x0, hx, object_columns);
@@ -385,7 +424,7 @@ __global__ void __launch_bounds__(256) tile_lists_kernel(const int *rr, const in
         }
         n += __popc(ballot);
     }
-    if (!list && lane == 0) counts[tile] = n;
+    if (!list && lane == 0) counts[part] = n;
 }
 
 // ------------------------------------------------------------------------------------------------ probe gather
@@ -780,14 +819,47 @@ cudaError_t launch_probe_gather_grouped(const ProbeGatherArgs<T> *args, const in
 }
 
 template <typename T>
-cudaError_t launch_object_gather(const ObjectGatherArgs<T> &a, int tiles, cudaStream_t s) {
+cudaError_t launch_object_gather(const ObjectGatherArgs<T> &a, int parts, cudaStream_t s) {
     if constexpr (std::is_same<T, double>::value) {
         if (a.states > 1) {  // the mixed-state form exists in FP64 only
-            object_gather_kernel<T, true><<<tiles, kGatherThreads, 0, s>>>(a);
+            object_gather_kernel<T, true><<<parts, kGatherThreads, 0, s>>>(a);
             return cudaGetLastError();
         }
     }
-    object_gather_kernel<T, false><<<tiles, kGatherThreads, 0, s>>>(a);
+    object_gather_kernel<T, false><<<parts, kGatherThreads, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t launch_object_combine(const ObjectGatherArgs<T> &a, cudaStream_t s) {
+    if (a.groups == 1) return cudaSuccess;
+    object_combine_kernel<T><<<object_combine_blocks(a.object_rows, a.object_columns), kGatherThreads, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+// One wave of gather CTAs (four per SM) is 592; a tile under the middle of the scan has every position of a window's area
+// in its list, one under the edge few, so an object of few tiles leaves most SMs waiting for the middle ones.  Splitting
+// each tile's candidates into groups whose sums are added afterwards shortens that tail.  Measured, ms per gather with 1,
+// 2, 4 and 8 groups: 3,364 positions of 128 x 128 (529 tiles) 0.353 0.253 0.202 0.193; 2,304 of 96 x 96 (324 tiles) 0.187
+// 0.114 0.084 0.080; 576 of 64 x 64 (100 tiles) 0.062 0.040 0.029 0.021; 4,096 of 256 x 256 (1,024 tiles) 1.02 0.68 0.62
+// 0.61; 1,600 of 128 x 128 in FP64, four states (324 tiles) 1.38, 8 groups 0.45; but 16,384 of 128 x 128 (1,600 tiles)
+// 0.681 0.736 0.745 0.675 and 40,000 (3,364 tiles) 1.50 1.51 1.52 1.55.  The number depends on the object and the position
+// count only, not on the tile shape, so every shape sums in the same order.
+int object_gather_groups(long long objects, int positions) {
+    const long long tiles = (objects + kGatherThreads - 1) / kGatherThreads;
+    if (tiles >= 1300) return 1;
+    return (int)std::max<long long>(1, std::min<long long>({8, (4096 + tiles - 1) / tiles, positions / 64}));
+}
+
+int object_combine_blocks(int object_rows, int object_columns) {
+    return (int)(((long long)object_rows * object_columns + kGatherThreads - 1) / kGatherThreads);
+}
+
+template <typename T>
+cudaError_t launch_object_combine_grouped(const ObjectGatherArgs<T> *args, const int *prefix, int items, int total,
+                                          cudaStream_t s) {
+    if (total <= 0) return cudaSuccess;
+    object_combine_grouped_kernel<T><<<total, kGatherThreads, 0, s>>>(args, prefix, items, total);
     return cudaGetLastError();
 }
 
@@ -845,10 +917,11 @@ cudaError_t launch_object_cap(C2<T> *object, int count, int pure_phase, cudaStre
 int error_reduce_scratch() { return kErrorBlocks; }
 
 cudaError_t launch_tile_lists(const int *rr, const int *cc, int count, int rows, int columns, int object_rows,
-                              int object_columns, int tile_w, int tile_h, int tiles_x, int tiles, int *counts,
-                              const int *starts, int *list, int capacity, cudaStream_t s) {
-    tile_lists_kernel<<<(tiles + 7) / 8, 256, 0, s>>>(rr, cc, count, rows, columns, object_rows, object_columns, tile_w,
-                                                      tile_h, tiles_x, tiles, counts, starts, list, capacity);
+                              int object_columns, int tile_w, int tile_h, int tiles_x, int tiles, int groups,
+                              int *counts, const int *starts, int *list, int capacity, cudaStream_t s) {
+    tile_lists_kernel<<<(tiles * groups + 7) / 8, 256, 0, s>>>(rr, cc, count, rows, columns, object_rows, object_columns,
+                                                               tile_w, tile_h, tiles_x, tiles, groups, counts, starts,
+                                                               list, capacity);
     return cudaGetLastError();
 }
 
@@ -877,9 +950,12 @@ cudaError_t launch_error_reduce(const double *error, long long count, double div
                                                          cudaStream_t);                                              \
     template cudaError_t launch_object_gather_grouped<T>(const ObjectGatherArgs<T> *, const int *, int, int,          \
                                                          cudaStream_t);                                              \
+    template cudaError_t launch_object_combine_grouped<T>(const ObjectGatherArgs<T> *, const int *, int, int,          \
+                                                          cudaStream_t);                                              \
     template cudaError_t launch_probe_gather_grouped<T>(const ProbeGatherArgs<T> *, const int *, int, int,            \
                                                         cudaStream_t);                                               \
     template cudaError_t launch_object_gather<T>(const ObjectGatherArgs<T> &, int, cudaStream_t);                      \
+    template cudaError_t launch_object_combine<T>(const ObjectGatherArgs<T> &, cudaStream_t);                          \
     template cudaError_t launch_probe_gather<T>(const ProbeGatherArgs<T> &, cudaStream_t);                             \
     template int probe_gather_resident_ctas<T>();                                                                      \
     template cudaError_t launch_probe_reduce<T>(const C2<T> *, const T *, int, int, double2 *, double *, double *,     \

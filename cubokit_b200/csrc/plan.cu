@@ -222,6 +222,8 @@ struct cubo_ptycho_plan {
     int classes = 1;        // shift classes; class 0 is the zero shift
     int groups = 1;         // probe-gather position groups
     int tiles_x = 0, tiles = 0;
+    int gather_groups = 1, gather_maxima = 0;  // shares of each tile's candidates; entries of tile_max per slice
+    DeviceBuffer gather_grad, gather_weight;   // their partial sums
     int tile_w = kTileW, tile_h = kTileH;  // object-gather tile
     int probe_blocks = 0;
     bool fast = false;      // 128 x 128 FP32 register-resident position pass
@@ -467,24 +469,32 @@ void build_scan(cubo_ptycho_plan *p, const double *rows_in, const double *column
     p->tiles_x = (p->OC + p->tile_w - 1) / p->tile_w;
     const int tiles_y = (p->OR + p->tile_h - 1) / p->tile_h;
     p->tiles = p->tiles_x * tiles_y;
+    p->gather_groups = object_gather_groups(p->objects, P);
+    p->gather_maxima = p->gather_groups > 1 ? object_combine_blocks(p->OR, p->OC) : p->tiles;
+    if (p->gather_groups > 1) {
+        const size_t values = (size_t)p->gather_groups * p->objects;
+        check(p->gather_grad.alloc(values * (p->fp64 ? sizeof(double2) : sizeof(float2))), "cudaMalloc gather groups");
+        check(p->gather_weight.alloc(values * (p->fp64 ? sizeof(double) : sizeof(float))), "cudaMalloc gather groups");
+    }
     {
+        const int parts = p->tiles * p->gather_groups;
         // counted and listed on the device from the wrapped centres (one warp per tile, positions ascending)
-        if (p->tile_start.bytes < (size_t)(p->tiles + 1) * sizeof(int))
-            check(p->tile_start.alloc((size_t)(p->tiles + 1) * sizeof(int)), "cudaMalloc");
+        if (p->tile_start.bytes < (size_t)(parts + 1) * sizeof(int))
+            check(p->tile_start.alloc((size_t)(parts + 1) * sizeof(int)), "cudaMalloc");
         check(launch_tile_lists(p->rr.as<int>(), p->cc.as<int>(), P, R, C, p->OR, p->OC, p->tile_w, p->tile_h, p->tiles_x,
-                                p->tiles, p->tile_start.as<int>(), nullptr, nullptr, 0, s), "count candidates");
-        std::vector<int> counts(p->tiles + 1, 0);
-        check(cudaMemcpyAsync(counts.data(), p->tile_start.ptr, (size_t)p->tiles * sizeof(int), cudaMemcpyDeviceToHost, s),
+                                p->tiles, p->gather_groups, p->tile_start.as<int>(), nullptr, nullptr, 0, s), "count candidates");
+        std::vector<int> counts(parts + 1, 0);
+        check(cudaMemcpyAsync(counts.data(), p->tile_start.ptr, (size_t)parts * sizeof(int), cudaMemcpyDeviceToHost, s),
               "download counts");
         check(cudaStreamSynchronize(s), "count candidates");
         long long total = 0;
-        for (int t = 0; t < p->tiles; t++) {  // exclusive sums
+        for (int t = 0; t < parts; t++) {  // exclusive sums
             const int c = counts[t];
             counts[t] = (int)total;
             total += c;
         }
         if (total > INT32_MAX) fail(CUBO_PTYCHO_UNSUPPORTED, "object-gather candidate lists exceed 2^31 entries");
-        counts[p->tiles] = (int)total;
+        counts[parts] = (int)total;
         upload(p->tile_start, counts, s);
         // with position correction the lists are rebuilt on the device: room for every window's largest tile count
         const long long capacity =
@@ -494,7 +504,7 @@ void build_scan(cubo_ptycho_plan *p, const double *rows_in, const double *column
             check(p->tile_list.alloc((size_t)std::max<long long>(capacity, 1) * sizeof(int)), "cudaMalloc");
         p->tile_capacity = std::max<long long>(capacity, 1);
         check(launch_tile_lists(p->rr.as<int>(), p->cc.as<int>(), P, R, C, p->OR, p->OC, p->tile_w, p->tile_h, p->tiles_x,
-                                p->tiles, nullptr, p->tile_start.as<int>(), p->tile_list.as<int>(),
+                                p->tiles, p->gather_groups, nullptr, p->tile_start.as<int>(), p->tile_list.as<int>(),
                                 (int)std::min<long long>(p->tile_capacity, INT32_MAX), s), "list candidates");
     }
     const size_t shifted_bytes = (size_t)p->states * p->classes * n * (p->fp64 ? sizeof(double2) : sizeof(float2));
@@ -516,20 +526,21 @@ void build_scan(cubo_ptycho_plan *p, const double *rows_in, const double *column
 }
 
 // Bands of an iteration run band by band (split-BF16): band b holds positions [b band_size, (b + 1) band_size).  Lists
-// per band the object-gather tiles with a candidate inside it (ascending), and every tile without candidates in band 0,
+// per band the object-gather parts (tile and group) with a candidate inside it (ascending), and every part without any in band 0,
 // which writes their zero sums and maxima.
 void build_band_tiles(cubo_ptycho_plan *p) {
     cudaStream_t s = p->ctx->stream;
-    std::vector<int> starts(p->tiles + 1), list;
+    const int parts = p->tiles * p->gather_groups;
+    std::vector<int> starts(parts + 1), list;
     check(cudaMemcpyAsync(starts.data(), p->tile_start.ptr, starts.size() * sizeof(int), cudaMemcpyDeviceToHost, s),
           "download candidate lists");
     check(cudaStreamSynchronize(s), "download candidate lists");
-    list.resize(std::max(1, starts[p->tiles]));
-    check(cudaMemcpyAsync(list.data(), p->tile_list.ptr, (size_t)starts[p->tiles] * sizeof(int), cudaMemcpyDeviceToHost,
+    list.resize(std::max(1, starts[parts]));
+    check(cudaMemcpyAsync(list.data(), p->tile_list.ptr, (size_t)starts[parts] * sizeof(int), cudaMemcpyDeviceToHost,
                           s), "download candidate lists");
     check(cudaStreamSynchronize(s), "download candidate lists");
     std::vector<std::vector<int>> per_band(p->bands);
-    for (int t = 0; t < p->tiles; t++) {
+    for (int t = 0; t < parts; t++) {
         if (starts[t] == starts[t + 1]) { per_band[0].push_back(t); continue; }
         int last = -1;
         for (int i = starts[t]; i < starts[t + 1]; i++) {  // candidates ascending: their bands too
@@ -600,7 +611,7 @@ void build_plan(cubo_ptycho_plan *p, const cubo_ptycho_problem *pr) {
     check(p->object.alloc((size_t)p->slices * p->objects * sizeof(C2<T>)), "cudaMalloc object");
     check(p->grad_o.alloc((size_t)p->slices * p->objects * sizeof(C2<T>)), "cudaMalloc");
     check(p->weight_o.alloc((size_t)p->slices * p->objects * sizeof(T)), "cudaMalloc");
-    check(p->tile_max.alloc((size_t)p->slices * p->tiles * sizeof(double)), "cudaMalloc");
+    check(p->tile_max.alloc((size_t)p->slices * p->gather_maxima * sizeof(double)), "cudaMalloc");
     if (p->multislice) {
         check(p->waves64.alloc((size_t)(p->slices - 1) * P * n * sizeof(double2)), "cudaMalloc entering waves");
         check(p->slice_max.alloc((size_t)p->slices * sizeof(double)), "cudaMalloc");
@@ -971,6 +982,7 @@ ObjectGatherArgs<T> object_gather_args(cubo_ptycho_plan *p) {
     ObjectGatherArgs<T> ga{};
     ga.rows = p->R; ga.columns = p->C; ga.object_rows = p->OR; ga.object_columns = p->OC; ga.n = n;
     ga.tiles_x = p->tiles_x; ga.tile_w = p->tile_w; ga.tile_h = p->tile_h; ga.tile_start = p->tile_start.as<int>(); ga.tile_list = p->tile_list.as<int>();
+    ga.groups = p->gather_groups; ga.part_grad = p->gather_grad.as<C2<T>>(); ga.part_weight = p->gather_weight.as<T>();
     ga.scan = ScanTables{p->rr.as<int>(), p->cc.as<int>(), p->cls.as<int>()};
     ga.shifted = p->shifted.as<C2<T>>(); ga.dpsi = p->dpsi.as<C2<T>>();
     ga.grad = p->grad_o.as<C2<T>>(); ga.weight = p->weight_o.as<T>(); ga.tile_max = p->tile_max.as<double>();
@@ -978,6 +990,13 @@ ObjectGatherArgs<T> object_gather_args(cubo_ptycho_plan *p) {
     ga.dpsi_state_stride = (long long)p->P * n;
     ga.shifted_state_stride = (long long)p->classes * n;
     return ga;
+}
+
+// The object gather over every tile and group, and the groups' sum.
+template <typename T>
+cudaError_t gather_object(const cubo_ptycho_plan *p, const ObjectGatherArgs<T> &ga) {
+    const cudaError_t e = launch_object_gather<T>(ga, p->tiles * p->gather_groups, p->ctx->stream);
+    return e == cudaSuccess ? launch_object_combine<T>(ga, p->ctx->stream) : e;
 }
 
 // The probe gather's arguments over every position of the plan (probe state 0).
@@ -997,7 +1016,7 @@ void enqueue_gathers(cubo_ptycho_plan *p) {
     ensure_dpsi<T>(p);
     const int n = p->n;
     const ObjectGatherArgs<T> ga = object_gather_args<T>(p);
-    if (!p->grouped_gathers) timed(p, kObjectGather, 1, [&] { return launch_object_gather<T>(ga, p->tiles, s); });
+    if (!p->grouped_gathers) timed(p, kObjectGather, p->gather_groups > 1 ? 2 : 1, [&] { return gather_object<T>(p, ga); });
 
     ProbeGatherArgs<T> pg = probe_gather_args<T>(p);
     for (int st = 0; st < p->states; st++) {  // each probe state's gradient from its own residuals
@@ -1011,7 +1030,7 @@ void enqueue_gathers(cubo_ptycho_plan *p) {
         });
     }
     timed(p, kMaxReduce, 2, [&] {
-        cudaError_t e = launch_max_reduce(p->tile_max.as<double>(), p->tiles, p->maxes.as<double>(), s);
+        cudaError_t e = launch_max_reduce(p->tile_max.as<double>(), p->gather_maxima, p->maxes.as<double>(), s);
         if (e == cudaSuccess) e = launch_max_reduce(p->probe_block_max.as<double>(), p->probe_blocks, p->maxes.as<double>() + 1, s);
         return e;
     });
@@ -1045,6 +1064,8 @@ void enqueue_banded_pass_and_gathers(cubo_ptycho_plan *p) {
     ga.rows = p->R; ga.columns = p->C; ga.object_rows = p->OR; ga.object_columns = p->OC; ga.n = n;
     ga.tiles_x = p->tiles_x; ga.tile_w = p->tile_w; ga.tile_h = p->tile_h;
     ga.tile_start = p->tile_start.as<int>(); ga.tile_list = p->tile_list.as<int>();
+    ga.groups = p->gather_groups; ga.part_grad = p->gather_grad.as<float2>();
+    ga.part_weight = p->gather_weight.as<float>();
     ga.scan = scan; ga.shifted = p->shifted.as<float2>(); ga.dpsi = p->dpsi_band.as<float2>();
     ga.grad = p->grad_o.as<float2>(); ga.weight = p->weight_o.as<float>(); ga.tile_max = p->tile_max.as<double>();
     ProbeGatherArgs<float> pg{};
@@ -1060,20 +1081,21 @@ void enqueue_banded_pass_and_gathers(cubo_ptycho_plan *p) {
             fa.first = first; fa.count = count; fa.dpsi_first = first; fa.accumulate = b > 0 ? 1 : 0;
             timed(p, kPositionPass, 1, [&] { return launch_fast128(fa, p->sms, s); });
         }
-        const int tiles = p->band_tile_offsets[b + 1] - p->band_tile_offsets[b];
+        const int parts = p->band_tile_offsets[b + 1] - p->band_tile_offsets[b];
         ga.band_tiles = p->band_tiles.as<int>() + p->band_tile_offsets[b];
         ga.band_first = first; ga.band_end = first + count;
-        if (tiles > 0) timed(p, kObjectGather, 1, [&] { return launch_object_gather<float>(ga, tiles, s); });
+        if (parts > 0) timed(p, kObjectGather, 1, [&] { return launch_object_gather<float>(ga, parts, s); });
         pg.first = first; pg.count = count; pg.accumulate = b > 0 ? 1 : 0;
         if (p->bf16) timed(p, kProbeGather, 1, [&] { return launch_probe_gather<float>(pg, s); });
     }
+    if (ga.groups > 1) timed(p, kObjectGather, 1, [&] { return launch_object_combine<float>(ga, s); });
     timed(p, kProbeReduce, 1, [&] {
         return launch_probe_reduce<float>(p->partial_grad.as<float2>(), p->partial_weight.as<float>(), p->groups, n,
                                           p->grad_p64.as<double2>(), p->weight_p64.as<double>(),
                                           p->probe_block_max.as<double>(), s);
     });
     timed(p, kMaxReduce, 2, [&] {
-        cudaError_t e = launch_max_reduce(p->tile_max.as<double>(), p->tiles, p->maxes.as<double>(), s);
+        cudaError_t e = launch_max_reduce(p->tile_max.as<double>(), p->gather_maxima, p->maxes.as<double>(), s);
         if (e == cudaSuccess) e = launch_max_reduce(p->probe_block_max.as<double>(), p->probe_blocks, p->maxes.as<double>() + 1, s);
         return e;
     });
@@ -1230,13 +1252,15 @@ void enqueue_multislice_iteration(cubo_ptycho_plan *p) {
     ga.rows = p->R; ga.columns = p->C; ga.object_rows = p->OR; ga.object_columns = p->OC; ga.n = n;
     ga.tiles_x = p->tiles_x; ga.tile_w = p->tile_w; ga.tile_h = p->tile_h;
     ga.tile_start = p->tile_start.as<int>(); ga.tile_list = p->tile_list.as<int>(); ga.dpsi = chi;
+    ga.groups = p->gather_groups; ga.part_grad = p->gather_grad.as<double2>();
+    ga.part_weight = p->gather_weight.as<double>();
     for (int sl = L - 1; sl >= 0; sl--) {
         ga.scan = sl == 0 ? scan : own;
         ga.shifted = sl == 0 ? shifted : waves + (size_t)(sl - 1) * planes;
         ga.grad = p->grad_o.as<double2>() + (size_t)sl * plane;
         ga.weight = p->weight_o.as<double>() + (size_t)sl * plane;
-        ga.tile_max = p->tile_max.as<double>() + (size_t)sl * p->tiles;
-        timed(p, kObjectGather, 1, [&] { return launch_object_gather<double>(ga, p->tiles, s); });
+        ga.tile_max = p->tile_max.as<double>() + (size_t)sl * p->gather_maxima;
+        timed(p, kObjectGather, p->gather_groups > 1 ? 2 : 1, [&] { return gather_object<double>(p, ga); });
         if (sl == 0) break;
         if (p->plane128) {
             enqueue_plane128(p, kBackPropagation, chi, false, obj + (size_t)sl * plane, true, false,
@@ -1264,7 +1288,7 @@ void enqueue_multislice_iteration(cubo_ptycho_plan *p) {
     timed(p, kMaxReduce, L + 1, [&] {
         cudaError_t e = cudaSuccess;
         for (int sl = 0; sl < L && e == cudaSuccess; sl++)
-            e = launch_max_reduce(p->tile_max.as<double>() + (size_t)sl * p->tiles, p->tiles,
+            e = launch_max_reduce(p->tile_max.as<double>() + (size_t)sl * p->gather_maxima, p->gather_maxima,
                                   p->slice_max.as<double>() + sl, s);
         if (e == cudaSuccess)
             e = launch_max_reduce(p->probe_block_max.as<double>(), p->probe_blocks, p->maxes.as<double>() + 1, s);
@@ -1347,8 +1371,8 @@ void refresh_scan(cubo_ptycho_plan *p) {
     if (!p->correct_positions || !p->scan_stale) return;
     cudaStream_t s = p->ctx->stream;
     const int P = p->P;
-    if (p->tile_counts.bytes < (size_t)p->tiles * sizeof(int))
-        check(p->tile_counts.alloc((size_t)p->tiles * sizeof(int)), "cudaMalloc");
+    if (p->tile_counts.bytes < (size_t)p->tiles * p->gather_groups * sizeof(int))
+        check(p->tile_counts.alloc((size_t)p->tiles * p->gather_groups * sizeof(int)), "cudaMalloc");
     timed(p, kPositionCorrection, 5, [&] {
         cudaError_t e = launch_scan_tables(p->positions64.as<double>(), P, p->OR, p->OC, p->rr.as<int>(),
                                            p->cc.as<int>(), p->cls.as<int>(), p->fractions64.as<double2>(), s);
@@ -1357,13 +1381,13 @@ void refresh_scan(cubo_ptycho_plan *p) {
                                   p->ramps_c64.as<double2>(), s);
         if (e == cudaSuccess)
             e = launch_tile_lists(p->rr.as<int>(), p->cc.as<int>(), P, p->R, p->C, p->OR, p->OC, p->tile_w, p->tile_h,
-                                  p->tiles_x, p->tiles, p->tile_counts.as<int>(), nullptr, nullptr, 0, s);
+                                  p->tiles_x, p->tiles, p->gather_groups, p->tile_counts.as<int>(), nullptr, nullptr, 0, s);
         if (e == cudaSuccess)
-            e = launch_exclusive_scan(p->tile_counts.as<int>(), p->tiles, p->tile_start.as<int>(), p->tile_capacity,
+            e = launch_exclusive_scan(p->tile_counts.as<int>(), p->tiles * p->gather_groups, p->tile_start.as<int>(), p->tile_capacity,
                                       p->position_bad.as<int>(), s);
         if (e == cudaSuccess)
             e = launch_tile_lists(p->rr.as<int>(), p->cc.as<int>(), P, p->R, p->C, p->OR, p->OC, p->tile_w, p->tile_h,
-                                  p->tiles_x, p->tiles, nullptr, p->tile_start.as<int>(), p->tile_list.as<int>(),
+                                  p->tiles_x, p->tiles, p->gather_groups, nullptr, p->tile_start.as<int>(), p->tile_list.as<int>(),
                                   (int)std::min<long long>(p->tile_capacity, INT32_MAX), s);
         return e;
     });
@@ -2102,7 +2126,7 @@ struct cubo_ptycho_batch {
     // argument structure per item and the items' unit offsets in device memory.
     struct Group {
         int wave = 0;  // the wave of items it belongs to
-        int kind = 0;  // 0 position pass, 1 object gather, 2 probe gather
+        int kind = 0;  // 0 position pass, 1 object gather, 2 probe gather, 3 the sum of the object gather's groups
         bool fp64 = false;
         int N = 0, shape = 0;
         std::vector<cubo_ptycho_plan *> plans;
@@ -2132,7 +2156,7 @@ void upload_group_args(cubo_ptycho_batch::Group &g, cudaStream_t s) {
         std::vector<PositionPassArgs<T>> v;
         for (auto *p : g.plans) v.push_back(position_pass_args<T>(p));
         upload(g.args, v, s);
-    } else if (g.kind == 1) {
+    } else if (g.kind == 1 || g.kind == 3) {
         std::vector<ObjectGatherArgs<T>> v;
         for (auto *p : g.plans) v.push_back(object_gather_args<T>(p));
         upload(g.args, v, s);
@@ -2193,7 +2217,8 @@ void build_groups(cubo_ptycho_batch *b) {
             add(0, p, p->R, p->params.pass_shape, p->P);
             p->grouped_pass = true;
         }
-        add(1, p, 0, 0, p->tiles);
+        add(1, p, 0, 0, p->tiles * p->gather_groups);
+        if (p->gather_groups > 1) add(3, p, 0, 0, p->gather_maxima);
         if (!p->fast) add(2, p, 0, 0, ((p->n + 255) / 256) * p->groups);
         p->grouped_gathers = true;
     }
@@ -2211,6 +2236,8 @@ cudaError_t launch_group(const cubo_ptycho_batch::Group &g, cudaStream_t s) {
                                                g.N, g.shape, s);
     if (g.kind == 1)
         return launch_object_gather_grouped<T>(g.args.as<ObjectGatherArgs<T>>(), g.offsets.as<int>(), items, total, s);
+    if (g.kind == 3)
+        return launch_object_combine_grouped<T>(g.args.as<ObjectGatherArgs<T>>(), g.offsets.as<int>(), items, total, s);
     return launch_probe_gather_grouped<T>(g.args.as<ProbeGatherArgs<T>>(), g.offsets.as<int>(), items, total, s);
 }
 
@@ -2236,7 +2263,7 @@ void capture_batch(cubo_ptycho_batch *b) {
                 else if (p->fp64) enqueue_position_pass<double>(p);
                 else enqueue_position_pass<float>(p);
             }
-            for (int kind = 0; kind < 3; kind++)  // the wave's passes before any of its gathers
+            for (int kind = 0; kind < 4; kind++)  // the wave's passes before any of its gathers
                 for (const auto &g : b->groups)
                     if (g->wave == w && g->kind == kind)
                         check(g->fp64 ? launch_group<double>(*g, s) : launch_group<float>(*g, s), "grouped launch");
