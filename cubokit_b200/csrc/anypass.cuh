@@ -25,6 +25,7 @@
 #pragma once
 
 #include "engine.h"
+#include "project.cuh"
 #include "regdft.cuh"
 
 namespace cubo {
@@ -172,19 +173,7 @@ __device__ __forceinline__ double centre_stage(C2<T> *D, const AnyPassArgs<T> &g
 #pragma unroll
         for (int r = 0; r < R; r++) x[r] = x0[r * g.pitch];
         regdft::dft<T, false, R>(x);
-#pragma unroll
-        for (int q = 0; q < R; q++) {
-            const T mag = sqrt(x[q].x * x[q].x + x[q].y * x[q].y);
-            const T want = (T)measured[q], miss = want - mag;
-            err += (double)(miss * miss);
-            if (mag > (T)0) {
-                const T s = (want / mag - (T)1) * a.inv_n;
-                x[q].x *= s;
-                x[q].y *= s;
-            } else {
-                x[q] = mk<T>(want * a.inv_n, (T)0);
-            }
-        }
+        project_values<T, R>(x, measured, a.inv_n, err);
         regdft::dft<T, true, R>(x);
 #pragma unroll
         for (int r = 0; r < R; r++) x0[r * g.pitch] = x[r];

@@ -17,6 +17,7 @@
 #include <type_traits>
 
 #include "engine.h"
+#include "project.cuh"
 
 namespace cubo {
 
@@ -181,17 +182,10 @@ __global__ void __launch_bounds__(NT) project_global_kernel(PositionPassArgs<dou
     const float *A = a.amplitudes + (size_t)p * a.n;
     double err = 0;
     for (int k = threadIdx.x; k < a.n; k += NT) {
-        const double2 f = D[k];
-        const double mag = sqrt(f.x * f.x + f.y * f.y);
-        const double measured = (double)A[k];
-        const double miss = measured - mag;
-        err += miss * miss;
-        if (mag > 0.0) {
-            const double sc = (measured / mag - 1.0) * a.inv_n;
-            D[k] = make_double2(f.x * sc, f.y * sc);
-        } else {
-            D[k] = make_double2(measured * a.inv_n, 0.0);
-        }
+        double2 f[1] = {D[k]};
+        const float measured[1] = {A[k]};
+        project_values<double, 1>(f, measured, a.inv_n, err);
+        D[k] = f[0];
     }
     const double total = block_sum<NT>(err, scratch);
     if (threadIdx.x == 0) a.error[p] = total;

@@ -150,8 +150,7 @@ __global__ void __launch_bounds__(kG32Threads, 4) g32_columns_fixed(const __grid
 #pragma unroll
             for (int r = 0; r < RB; r++) x[r] = y[r * NL];
             regdft::dft<float, false, RB>(x);
-#pragma unroll
-            for (int q = 0; q < RB; q++) x[q] = g32_project(x[q], measured[q], a.inv_n, err);
+            project_values<float, RB>(x, measured, a.inv_n, err);
             regdft::dft<float, true, RB>(x);
 #pragma unroll
             for (int r = 0; r < RB; r++) y[r * NL] = x[r];
@@ -225,7 +224,10 @@ __global__ void __launch_bounds__(kG32Threads, 2) g32_columns_direct(PositionPas
     double err = 0;
     for (int i = threadIdx.x; i < nl * L; i += kG32Threads) {
         const int e = i / nl, j = i - e * nl;
-        D[i] = g32_project(D[i], A[(size_t)e * a.columns + j], a.inv_n, err);
+        float2 f[1] = {D[i]};
+        const float measured[1] = {A[(size_t)e * a.columns + j]};
+        project_values<float, 1>(f, measured, a.inv_n, err);
+        D[i] = f[0];
     }
     const double total = g32_block_sum(err, scratch);  // its barriers also order the projection before the inverse
     if (threadIdx.x == 0) a.error[(size_t)p * per + c0 / nl] = total;

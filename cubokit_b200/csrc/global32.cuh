@@ -217,18 +217,6 @@ __global__ void __launch_bounds__(kG32Threads, WIDE ? 1 : 4) g32_rows_inverse(co
 
 // ------------------------------------------------------------------------------------------- columns, run-time plan
 
-// The projection of one far-field value (Ptychography.swift:338-349); adds its squared residual.
-__device__ __forceinline__ float2 g32_project(float2 f, float measured, float inv_n, double &err) {
-    const float mag = sqrtf(f.x * f.x + f.y * f.y);
-    const float miss = measured - mag;
-    err += (double)(miss * miss);
-    if (mag > 0.f) {
-        const float s = (measured / mag - 1.f) * inv_n;
-        return make_float2(f.x * s, f.y * s);
-    }
-    return make_float2(measured * inv_n, 0.f);
-}
-
 // Columns c0 .. of position p, sample e of column c at D[e nl + c].  The CTA's squared residual goes to
 // error[p per + c0 / nl].
 template <bool WIDE>
@@ -293,8 +281,7 @@ __global__ void __launch_bounds__(kG32Threads, WIDE ? 1 : 4) g32_columns(const _
 #pragma unroll
             for (int r = 0; r < R; r++) x[r] = y[(size_t)r * step];
             regdft::dft<float, false, R>(x);
-#pragma unroll
-            for (int q = 0; q < R; q++) x[q] = g32_project(x[q], measured[q], a.inv_n, err);
+            project_values<float, R>(x, measured, a.inv_n, err);
             regdft::dft<float, true, R>(x);
 #pragma unroll
             for (int r = 0; r < R; r++) y[(size_t)r * step] = x[r];

@@ -14,6 +14,7 @@
 #include <cfloat>
 
 #include "engine.h"
+#include "project.cuh"
 
 namespace cubo {
 
@@ -70,9 +71,14 @@ __global__ void __launch_bounds__(kProjectThreads) mixed_project_kernel(double2 
             const double2 f = dpsi[((size_t)s * count + p) * n + k];
             intensity += f.x * f.x + f.y * f.y;
         }
-        const double amplitude = sqrt(intensity), measured = (double)A[k];
+        const double measured = (double)A[k];
         double factor;
-        if (amplitude == 0.0) {
+        if (modulus_in_range<double>(intensity, measured)) {
+            double amplitude, ratio;
+            modulus_and_ratio(intensity, measured, amplitude, ratio);
+            err += (measured - amplitude) * (measured - amplitude);
+            factor = (ratio - 1.0) * inv_n;
+        } else if (const double amplitude = sqrt(intensity); amplitude == 0.0) {
             err += zero_infinite ? (double)INFINITY : measured * measured;
             factor = 0.0;
         } else {

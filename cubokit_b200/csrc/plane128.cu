@@ -22,6 +22,7 @@
 
 #include "engine.h"
 #include "position_step.cuh"
+#include "project.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -446,22 +447,19 @@ __global__ void __cluster_dims__(Q, 1, 1) __launch_bounds__(PlaneGeometry<Q>::kT
             landed = mbarrier_wait_bounded(amp_ready);
         }
 #pragma unroll
-        for (int k2 = 0; k2 < 8; k2++)
+        for (int half = 0; half < 2; half++) {  // eight values at a time
+            double2 f[8];
+            float measured[8];
 #pragma unroll
-            for (int c = 0; c < 2; c++) {
-                const int kr = 2 * j + c + 16 * k2;
-                const double2 f = v[2 * k2 + c];
-                const double mag = sqrt(f.x * f.x + f.y * f.y);
-                const double measured = (double)amp[kr * G::kAmpStride + line];
-                const double miss = measured - mag;
-                err += miss * miss;
-                if (mag > 0.0) {
-                    const double sc = (measured / mag - 1.0) * a.inv_n;
-                    v[2 * k2 + c] = make_double2(f.x * sc, f.y * sc);
-                } else {
-                    v[2 * k2 + c] = make_double2(measured * a.inv_n, 0.0);
-                }
+            for (int i = 0; i < 8; i++) {
+                const int at = 8 * half + i;
+                f[i] = v[at];
+                measured[i] = amp[(2 * j + (at & 1) + 16 * (at >> 1)) * G::kAmpStride + line];
             }
+            project_values<double, 8>(f, measured, a.inv_n, err);
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[8 * half + i] = f[i];
+        }
     } else if (stage_factor) {  // the mixed states' common factor of each pixel (a real scale)
         bool landed = mbarrier_wait_bounded(amp_ready);
         if (!landed) {

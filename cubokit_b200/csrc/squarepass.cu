@@ -15,6 +15,7 @@
 // register-resident line transforms, two CTAs per SM: 96 x 96 0.577 -> 0.258 ms (57 -> 129 Gpixel/s), 64 x 64 0.201 ->
 // 0.109 ms (73 -> 135).
 #include "engine.h"
+#include "project.cuh"
 #include "regdft.cuh"
 
 namespace cubo {
@@ -115,19 +116,7 @@ __device__ __forceinline__ void square_pass_body(const PositionPassArgs<float> &
 #pragma unroll
             for (int r = 0; r < RA; r++) x[r] = x0[r * P];
             regdft::dft<float, false, RA>(x);
-#pragma unroll
-            for (int q = 0; q < RA; q++) {
-                const float mag = sqrtf(x[q].x * x[q].x + x[q].y * x[q].y);
-                const float miss = measured[q] - mag;
-                err += (double)(miss * miss);
-                if (mag > 0.f) {
-                    const float s = (measured[q] / mag - 1.f) * a.inv_n;
-                    x[q].x *= s;
-                    x[q].y *= s;
-                } else {
-                    x[q] = make_float2(measured[q] * a.inv_n, 0.f);
-                }
-            }
+            project_values<float, RA>(x, measured, a.inv_n, err);
             regdft::dft<float, true, RA>(x);
 #pragma unroll
             for (int r = 0; r < RA; r++) x0[r * P] = x[r];
