@@ -74,14 +74,14 @@ struct ProbeGatherArgs {
     int accumulate = 0;
 };
 
-// The 128 x 128 FP32 position pass (fast128.cu); amplitudes in its register order, 32 residual partials per position.
+// The 128 x 128 FP32 position pass (fast128.cu); amplitudes in its threads' order.
 struct Fast128Args {
     int object_rows, object_columns;
     int first, count;
     ScanTables scan;
     const float2 *shifted;
     const float2 *object;
-    const float *amplitudes;   // [positions][column][h][t][e] (fast128.cu)
+    const float *amplitudes;   // [positions][h][thread][e] (fast128.cu)
     float2 *dpsi;              // [positions - dpsi_first][row][column]
     int dpsi_first;            // the position whose residual dpsi[0] holds (a band's first, or 0)
     double *error;             // [positions][fast128_partials_per_position()]
@@ -89,7 +89,6 @@ struct Fast128Args {
     float2 *partial_grad;      // [fast128_ctas()][n] probe-gradient partials, one per CTA
     float *partial_weight;     // [fast128_ctas()][n]
     int accumulate;            // 1: each CTA's partial continues from the one it left (an earlier band), 0: from zero
-    int *fault;                // set when the amplitude prefetch wait ran out
 };
 int fast128_ctas();
 bool fast128_applicable(int rows, int columns);

@@ -631,7 +631,7 @@ void build_plan(cubo_ptycho_plan *p, const cubo_ptycho_problem *pr) {
                      : p->bf16     ? (long long)P * bf16_partials_per_position()
                      : p->global32 ? (long long)P * global32_partials_per_position(p->R, p->C)
                                    : P;
-    if (p->fast || p->plane128) {
+    if (p->plane128) {
         check(p->fault.alloc(sizeof(int)), "cudaMalloc");
         check(cudaMemsetAsync(p->fault.ptr, 0, sizeof(int), s), "memset");
     }
@@ -708,7 +708,7 @@ Fft2Plan64 fft64(const cubo_ptycho_plan *p) {
 
 // After a synchronize: a device wait that ran out (split-BF16 kernel) turns into CUBO_PTYCHO_DEVICE_TIMEOUT.
 void check_fault(cubo_ptycho_plan *p) {
-    if (!p->bf16 && !p->fast && !p->plane128) return;
+    if (!p->bf16 && !p->plane128) return;
     int f = 0;
     check(cudaMemcpy(&f, p->fault.ptr, sizeof(int), cudaMemcpyDeviceToHost), "read fault flag");
     if (f) {
@@ -916,7 +916,6 @@ void enqueue_position_pass(cubo_ptycho_plan *p) {
         fa.accumulate = 0; fa.error = p->error.as<double>();
         fa.tw128 = p->tw_r.as<float2>();
         fa.partial_grad = p->partial_grad.as<float2>(); fa.partial_weight = p->partial_weight.as<float>();
-        fa.fault = p->fault.as<int>();
         timed(p, kPositionPass, 1, [&] { return launch_fast128(fa, p->sms, s); });
     } else if (p->states > 1 && p->plane128) {
         if constexpr (std::is_same<T, double>::value) {  // every state's far field, the summed projection, inverses
@@ -1054,7 +1053,6 @@ void enqueue_banded_pass_and_gathers(cubo_ptycho_plan *p) {
     fa.amplitudes = p->amplitudes.as<float>(); fa.dpsi = p->dpsi_band.as<float2>(); fa.error = p->error.as<double>();
     fa.tw128 = p->tw_r.as<float2>();
     fa.partial_grad = p->partial_grad.as<float2>(); fa.partial_weight = p->partial_weight.as<float>();
-    fa.fault = p->fault.as<int>();
     Bf16Args ba{};
     ba.object_rows = p->OR; ba.object_columns = p->OC; ba.scan = scan;
     ba.shifted = p->shifted.as<float2>(); ba.object = p->object.as<float2>();
