@@ -69,10 +69,16 @@ SIGNATURES = {
     "cubo_ptycho_destroy": (C.c_int, [C.c_void_p]),
     "cubo_ptycho_last_error": (C.c_char_p, [C.c_void_p]),
     "cubo_ptycho_reconstruct": (C.c_int, [C.c_void_p, C.POINTER(Problem), C.POINTER(Params), _dp, _dp, _dp, _dp, _dp]),
+    "cubo_ptycho_reconstruct_complex": (C.c_int, [C.c_void_p, C.POINTER(Problem), C.POINTER(Params), _dp, _dp, _dp]),
     "cubo_ptycho_plan_create": (C.c_int, [C.c_void_p, C.POINTER(Problem), C.POINTER(Params), C.POINTER(C.c_void_p)]),
     "cubo_ptycho_plan_destroy": (C.c_int, [C.c_void_p]),
     "cubo_ptycho_plan_set_state": (C.c_int, [C.c_void_p, _dp, _dp, _dp, _dp]),
     "cubo_ptycho_plan_get_state": (C.c_int, [C.c_void_p, _dp, _dp, _dp, _dp]),
+    "cubo_ptycho_plan_set_state_complex": (C.c_int, [C.c_void_p, _dp, _dp]),
+    "cubo_ptycho_plan_get_state_complex": (C.c_int, [C.c_void_p, _dp, _dp]),
+    "cubo_ptycho_plan_backward_complex": (C.c_int, [C.c_void_p, C.c_int, _dp, _dp, _dp]),
+    "cubo_ptycho_batch_set_state_complex": (C.c_int, [C.c_void_p, C.c_int, _dp, _dp]),
+    "cubo_ptycho_batch_get_state_complex": (C.c_int, [C.c_void_p, C.c_int, _dp, _dp]),
     "cubo_ptycho_plan_get_positions": (C.c_int, [C.c_void_p, _dp, _dp]),
     "cubo_ptycho_mixed_params_default": (None, [C.POINTER(MixedParams)]),
     "cubo_ptycho_mixed_reconstruct": (C.c_int, [C.c_void_p, C.POINTER(Problem), C.POINTER(Params),

@@ -1,6 +1,7 @@
 // Host side of the engine: the C ABI of include/cubo_ptycho.h, input validation, the scan tables, device buffers and
 // the per-iteration launch sequence.  Runs on the caller's thread; all device work goes to the context's stream.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <functional>
 #include <limits>
@@ -16,6 +17,8 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "../../include/cubo_ptycho.h"
@@ -208,6 +211,134 @@ void *pinned_staging(cubo_ptycho_context *ctx, size_t bytes) {
     }
     return ctx->pinned;
 }
+
+namespace {
+
+// body(first, last) over `count` items in ranges of at least `grain` on up to eight host threads, the caller's among them
+// (a thread costs about 20 us to start; a complex value takes about 2 ns to convert on one).  body must not throw.
+template <typename F>
+void parallel_ranges(size_t count, size_t grain, const F &body) {
+    const size_t most = std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
+    const size_t parts = std::max<size_t>(1, std::min(most, count / grain));
+    std::vector<std::thread> threads;
+    size_t started = 1;
+    try {
+        threads.reserve(parts);
+        for (; started < parts; started++)
+            threads.emplace_back([&body, count, parts, part = started] {
+                body(count * part / parts, count * (part + 1) / parts);
+            });
+    } catch (const std::system_error &) {  // no more threads: the caller does the rest
+    }
+    body(0, count / parts);
+    for (size_t part = started; part < parts; part++) body(count * part / parts, count * (part + 1) / parts);
+    for (auto &t : threads) t.join();
+}
+
+constexpr size_t kConvertGrain = 1 << 16;  // values
+
+// The caller's complex arrays: a real and an imaginary plane (stride 1) or interleaved pairs (stride 2).
+struct ComplexIn {
+    const double *re, *im;
+    int stride;
+};
+struct ComplexOut {
+    double *re, *im;  // either may be null
+    int stride;
+};
+ComplexIn interleaved(const double *z) { return ComplexIn{z, z ? z + 1 : nullptr, 2}; }
+ComplexOut interleaved(double *z) { return ComplexOut{z, z ? z + 1 : nullptr, 2}; }
+
+// out[j] = in[j]; false if any value is not finite.
+template <typename V>
+bool convert_in(const ComplexIn &in, V *out, size_t count) {
+    using R = decltype(V::x);
+    std::atomic<bool> finite{true};
+    parallel_ranges(count, kConvertGrain, [&](size_t first, size_t last) {
+        bool ok = true;
+        auto run = [&](auto stride) {
+            constexpr size_t S = decltype(stride)::value;
+            for (size_t j = first; j < last; j++) {
+                const double re = in.re[S * j], im = in.im[S * j];
+                ok = ok && std::isfinite(re) && std::isfinite(im);
+                out[j].x = (R)re;
+                out[j].y = (R)im;
+            }
+        };
+        if (in.stride == 1) run(std::integral_constant<size_t, 1>());
+        else run(std::integral_constant<size_t, 2>());
+        if (!ok) finite = false;
+    });
+    return finite;
+}
+
+// out[j] = scale * in[j].
+template <typename V>
+void convert_out(const V *in, size_t count, double scale, const ComplexOut &out) {
+    parallel_ranges(count, kConvertGrain, [&](size_t first, size_t last) {
+        if (out.stride == 2 && out.re) {
+            for (size_t j = first; j < last; j++) {
+                out.re[2 * j] = scale * (double)in[j].x;
+                out.re[2 * j + 1] = scale * (double)in[j].y;
+            }
+            return;
+        }
+        if (out.re)
+            for (size_t j = first; j < last; j++) out.re[j] = scale * (double)in[j].x;
+        if (out.im)
+            for (size_t j = first; j < last; j++) out.im[j] = scale * (double)in[j].y;
+    });
+}
+
+// Copies `bytes` of host memory to the device.  Page-locked memory goes as it is; pageable memory of some size through
+// page-locked pieces that several threads fill while earlier ones travel (the driver's own staging is one thread: 9.4 MB of
+// amplitudes took 1.2 ms, this way 0.4).
+void upload_host(cubo_ptycho_context *ctx, void *dst, const void *src, size_t bytes) {
+    constexpr size_t kPiece = 1 << 20, kLeast = 4 << 20, kThreads = 8;
+    cudaPointerAttributes at{};
+    const bool known = cudaPointerGetAttributes(&at, src) == cudaSuccess;
+    if (!known) (void)cudaGetLastError();
+    if (bytes < kLeast || (known && at.type != cudaMemoryTypeUnregistered)) {
+        check(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream), "upload");
+        return;
+    }
+    // two pieces per thread; the staging buffer may still feed earlier copies of this stream
+    check(cudaStreamSynchronize(ctx->stream), "sync");
+    uint8_t *stage = static_cast<uint8_t *>(pinned_staging(ctx, 2 * kThreads * kPiece));
+    cudaEvent_t events[2 * kThreads] = {};
+    cudaError_t failed = cudaSuccess;
+    for (auto &e : events)
+        if (failed == cudaSuccess) failed = cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+    const size_t pieces = (bytes + kPiece - 1) / kPiece;
+    std::atomic<size_t> next{0};
+    std::atomic<int> error{(int)failed};
+    if (failed == cudaSuccess)
+        parallel_ranges(kThreads, 1, [&](size_t first, size_t last) {
+            cudaError_t e = cudaSetDevice(ctx->device);
+            for (size_t turn = 0; e == cudaSuccess && error == 0; turn++) {
+                const size_t piece = next++;
+                if (piece >= pieces) break;
+                // ranges are one slot pair each, or several where fewer threads run
+                const size_t slot = 2 * first + turn % (2 * (last - first));
+                uint8_t *at_piece = stage + slot * kPiece;
+                const size_t off = piece * kPiece, size = std::min(kPiece, bytes - off);
+                if (turn >= 2 * (last - first)) e = cudaEventSynchronize(events[slot]);
+                std::memcpy(at_piece, static_cast<const uint8_t *>(src) + off, size);
+                if (e == cudaSuccess)
+                    e = cudaMemcpyAsync(static_cast<uint8_t *>(dst) + off, at_piece, size, cudaMemcpyHostToDevice,
+                                        ctx->stream);
+                if (e == cudaSuccess) e = cudaEventRecord(events[slot], ctx->stream);
+            }
+            if (e != cudaSuccess) error = (int)e;
+        });
+    const cudaError_t done = cudaStreamSynchronize(ctx->stream);  // the pieces are free again
+    for (auto &e : events)
+        if (e) cudaEventDestroy(e);
+    check((cudaError_t)error.load(), "upload");
+    check(done, "upload");
+}
+
+}  // namespace
 
 // ------------------------------------------------------------------------------------------------ the plan
 
@@ -574,9 +705,10 @@ void build_plan(cubo_ptycho_plan *p, const cubo_ptycho_problem *pr) {
     build_scan(p, pr->position_rows, pr->position_columns);
     // ---- amplitudes (Float32, [position][row][column]; the 128 x 128 kernel's register order when it runs)
     check(p->amplitudes.alloc((size_t)P * n * sizeof(float)), "cudaMalloc amplitudes");
-    check(cudaMemcpyAsync(p->amplitudes.ptr, pr->amplitudes, (size_t)P * n * sizeof(float),
-                          pr->amplitudes_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s),
-          "upload amplitudes");
+    if (pr->amplitudes_on_device)
+        check(cudaMemcpyAsync(p->amplitudes.ptr, pr->amplitudes, (size_t)P * n * sizeof(float), cudaMemcpyDeviceToDevice, s),
+              "copy amplitudes");
+    else upload_host(p->ctx, p->amplitudes.ptr, pr->amplitudes, (size_t)P * n * sizeof(float));
     {
         // every amplitude finite and non-negative, and sum A^2 (Ptychography.swift:247-259), in the supplied order
         DeviceBuffer scratch, bad;
@@ -1822,35 +1954,29 @@ int cubo_ptycho_plan_destroy(cubo_ptycho_plan *plan) {
     return CUBO_PTYCHO_OK;
 }
 
-int cubo_ptycho_plan_set_state(cubo_ptycho_plan *p, const double *ore, const double *oim, const double *pre,
-                               const double *pim) {
+}  // extern "C"
+
+namespace {
+int set_state(cubo_ptycho_plan *p, const ComplexIn &object, const ComplexIn &probe) {
     if (!p) return CUBO_PTYCHO_INVALID_INPUT;
     return run_guarded(p->ctx, [&] {
-        if (!ore || !oim || !pre || !pim) fail(CUBO_PTYCHO_INVALID_INPUT, "null state");
-        const long long object_values = (long long)p->slices * p->objects;  // every slice, [slice][row][column]
-        for (long long j = 0; j < object_values; j++)
-            if (!std::isfinite(ore[j]) || !std::isfinite(oim[j])) fail(CUBO_PTYCHO_INVALID_INPUT, "object not finite");
-        const size_t probe_values = (size_t)p->states * p->n;  // every probe state, [state][row][column]
-        for (size_t k = 0; k < probe_values; k++)
-            if (!std::isfinite(pre[k]) || !std::isfinite(pim[k])) fail(CUBO_PTYCHO_INVALID_INPUT, "probe not finite");
+        if (!object.re || !object.im || !probe.re || !probe.im) fail(CUBO_PTYCHO_INVALID_INPUT, "null state");
+        const size_t object_values = (size_t)p->slices * p->objects;  // every slice, [slice][row][column]
+        const size_t probe_values = (size_t)p->states * p->n;         // every probe state, [state][row][column]
         cudaStream_t s = p->ctx->stream;
-        p->tape_valid = false;
         // through the context's pinned staging buffer: the probe (complex128), then the object in the plan's type
-        const size_t object_bytes = (size_t)object_values * (p->fp64 ? sizeof(double2) : sizeof(float2));
+        const size_t object_bytes = object_values * (p->fp64 ? sizeof(double2) : sizeof(float2));
         uint8_t *stage = static_cast<uint8_t *>(pinned_staging(p->ctx, probe_values * sizeof(double2) + object_bytes));
-        double2 *probe = reinterpret_cast<double2 *>(stage);
-        for (size_t k = 0; k < probe_values; k++) probe[k] = make_double2(pre[k], pim[k]);
-        if (p->fp64) {
-            double2 *o = reinterpret_cast<double2 *>(stage + probe_values * sizeof(double2));
-            for (long long j = 0; j < object_values; j++) o[j] = make_double2(ore[j], oim[j]);
-        } else {
-            float2 *o = reinterpret_cast<float2 *>(stage + probe_values * sizeof(double2));
-            for (long long j = 0; j < p->objects; j++) o[j] = make_float2((float)ore[j], (float)oim[j]);
-        }
-        check(cudaMemcpyAsync(p->probe64.ptr, probe, probe_values * sizeof(double2), cudaMemcpyHostToDevice, s),
+        uint8_t *object_stage = stage + probe_values * sizeof(double2);
+        const bool finite = p->fp64 ? convert_in(object, reinterpret_cast<double2 *>(object_stage), object_values)
+                                    : convert_in(object, reinterpret_cast<float2 *>(object_stage), object_values);
+        if (!finite) fail(CUBO_PTYCHO_INVALID_INPUT, "object not finite");
+        if (!convert_in(probe, reinterpret_cast<double2 *>(stage), probe_values))
+            fail(CUBO_PTYCHO_INVALID_INPUT, "probe not finite");
+        p->tape_valid = false;
+        check(cudaMemcpyAsync(p->probe64.ptr, stage, probe_values * sizeof(double2), cudaMemcpyHostToDevice, s),
               "upload probe");
-        check(cudaMemcpyAsync(p->object.ptr, stage + probe_values * sizeof(double2), object_bytes,
-                              cudaMemcpyHostToDevice, s), "upload object");
+        check(cudaMemcpyAsync(p->object.ptr, object_stage, object_bytes, cudaMemcpyHostToDevice, s), "upload object");
         check(cudaStreamSynchronize(s), "sync");
         // the initial Fourier amplitude for fixProbeAperture (PtychographyConstraints.swift:79-83)
         if (p->params.fix_probe_aperture) {
@@ -1862,29 +1988,44 @@ int cubo_ptycho_plan_set_state(cubo_ptycho_plan *p, const double *ore, const dou
     });
 }
 
-int cubo_ptycho_plan_get_state(cubo_ptycho_plan *p, double *ore, double *oim, double *pre, double *pim) {
+int get_state(cubo_ptycho_plan *p, const ComplexOut &object, const ComplexOut &probe) {
     if (!p) return CUBO_PTYCHO_INVALID_INPUT;
     return run_guarded(p->ctx, [&] {
         cudaStream_t s = p->ctx->stream;
         const size_t probe_values = (size_t)p->states * p->n;
-        const size_t object_values = p->fp64 ? (size_t)p->slices * p->objects : (size_t)p->objects;
+        const size_t object_values = (size_t)p->slices * p->objects;
         const size_t object_bytes = object_values * (p->fp64 ? sizeof(double2) : sizeof(float2));
         uint8_t *stage = static_cast<uint8_t *>(pinned_staging(p->ctx, probe_values * sizeof(double2) + object_bytes));
-        const double2 *probe = reinterpret_cast<const double2 *>(stage);
+        const uint8_t *object_stage = stage + probe_values * sizeof(double2);
         check(cudaMemcpyAsync(stage, p->probe64.ptr, probe_values * sizeof(double2), cudaMemcpyDeviceToHost, s),
               "download probe");
         check(cudaMemcpyAsync(stage + probe_values * sizeof(double2), p->object.ptr, object_bytes,
                               cudaMemcpyDeviceToHost, s), "download object");
         check(cudaStreamSynchronize(s), "sync");
-        if (p->fp64) {
-            const double2 *o = reinterpret_cast<const double2 *>(stage + probe_values * sizeof(double2));
-            for (size_t j = 0; j < object_values; j++) { if (ore) ore[j] = o[j].x; if (oim) oim[j] = o[j].y; }
-        } else {
-            const float2 *o = reinterpret_cast<const float2 *>(stage + probe_values * sizeof(double2));
-            for (size_t j = 0; j < object_values; j++) { if (ore) ore[j] = o[j].x; if (oim) oim[j] = o[j].y; }
-        }
-        for (size_t k = 0; k < probe_values; k++) { if (pre) pre[k] = probe[k].x; if (pim) pim[k] = probe[k].y; }
+        if (p->fp64) convert_out(reinterpret_cast<const double2 *>(object_stage), object_values, 1.0, object);
+        else convert_out(reinterpret_cast<const float2 *>(object_stage), object_values, 1.0, object);
+        convert_out(reinterpret_cast<const double2 *>(stage), probe_values, 1.0, probe);
     });
+}
+}  // namespace
+
+extern "C" {
+
+int cubo_ptycho_plan_set_state(cubo_ptycho_plan *p, const double *ore, const double *oim, const double *pre,
+                               const double *pim) {
+    return set_state(p, ComplexIn{ore, oim, 1}, ComplexIn{pre, pim, 1});
+}
+
+int cubo_ptycho_plan_set_state_complex(cubo_ptycho_plan *p, const double *object, const double *probe) {
+    return set_state(p, interleaved(object), interleaved(probe));
+}
+
+int cubo_ptycho_plan_get_state(cubo_ptycho_plan *p, double *ore, double *oim, double *pre, double *pim) {
+    return get_state(p, ComplexOut{ore, oim, 1}, ComplexOut{pre, pim, 1});
+}
+
+int cubo_ptycho_plan_get_state_complex(cubo_ptycho_plan *p, double *object, double *probe) {
+    return get_state(p, interleaved(object), interleaved(probe));
 }
 
 int cubo_ptycho_plan_get_positions(cubo_ptycho_plan *p, double *rows, double *columns) {
@@ -1984,25 +2125,41 @@ int cubo_ptycho_plan_iterate(cubo_ptycho_plan *p, int iterations, double *errors
     return status;
 }
 
-int cubo_ptycho_reconstruct(cubo_ptycho_context *ctx, const cubo_ptycho_problem *pr, const cubo_ptycho_params *pp,
-                            double *ore, double *oim, double *pre, double *pim, double *errors) {
+}  // extern "C"
+
+namespace {
+int reconstruct(cubo_ptycho_context *ctx, const cubo_ptycho_problem *pr, const cubo_ptycho_params *pp,
+                const ComplexOut &object, const ComplexOut &probe, double *errors) {
     if (!ctx) return CUBO_PTYCHO_INVALID_INPUT;
-    if (!ore || !oim || !pre || !pim || (pp && pp->iterations > 0 && !errors)) {
+    if (!object.re || !object.im || !probe.re || !probe.im || (pp && pp->iterations > 0 && !errors)) {
         ctx->last_error = "null output";
         return CUBO_PTYCHO_INVALID_INPUT;
     }
     cubo_ptycho_plan *plan = nullptr;
     int status = cubo_ptycho_plan_create(ctx, pr, pp, &plan);
     if (status != CUBO_PTYCHO_OK) return status;
-    status = cubo_ptycho_plan_set_state(plan, ore, oim, pre, pim);
+    status = set_state(plan, ComplexIn{object.re, object.im, object.stride}, ComplexIn{probe.re, probe.im, probe.stride});
     if (status == CUBO_PTYCHO_OK) status = cubo_ptycho_plan_iterate(plan, pp->iterations, errors);
-    if (status == CUBO_PTYCHO_OK) status = cubo_ptycho_plan_get_state(plan, ore, oim, pre, pim);
+    if (status == CUBO_PTYCHO_OK) status = get_state(plan, object, probe);
     if (status == CUBO_PTYCHO_OK && pp->position_rows_out && pp->position_columns_out)
         status = cubo_ptycho_plan_get_positions(plan, pp->position_rows_out, pp->position_columns_out);
     const std::string message = ctx->last_error;
     cubo_ptycho_plan_destroy(plan);
     ctx->last_error = message;
     return status;
+}
+}  // namespace
+
+extern "C" {
+
+int cubo_ptycho_reconstruct(cubo_ptycho_context *ctx, const cubo_ptycho_problem *pr, const cubo_ptycho_params *pp,
+                            double *ore, double *oim, double *pre, double *pim, double *errors) {
+    return reconstruct(ctx, pr, pp, ComplexOut{ore, oim, 1}, ComplexOut{pre, pim, 1}, errors);
+}
+
+int cubo_ptycho_reconstruct_complex(cubo_ptycho_context *ctx, const cubo_ptycho_problem *pr,
+                                    const cubo_ptycho_params *pp, double *object, double *probe, double *errors) {
+    return reconstruct(ctx, pr, pp, interleaved(object), interleaved(probe), errors);
 }
 
 }  // extern "C"
@@ -2020,16 +2177,41 @@ void enqueue_forward(cubo_ptycho_plan *p) {
     });
 }
 
+// The tape's gradients: the object's (scaled) and the probe's, and the loss.
 template <typename T>
-void download_object_gradient(cubo_ptycho_plan *p, double scale, double *re, double *im) {
-    std::vector<C2<T>> g((size_t)p->objects);
-    check(cudaMemcpyAsync(g.data(), p->grad_o.ptr, g.size() * sizeof(C2<T>), cudaMemcpyDeviceToHost, p->ctx->stream),
+void download_gradients(cubo_ptycho_plan *p, double scale, const ComplexOut &object, const ComplexOut &probe,
+                        double *loss) {
+    cudaStream_t s = p->ctx->stream;
+    const size_t probe_bytes = (size_t)p->n * sizeof(double2), object_bytes = (size_t)p->objects * sizeof(C2<T>);
+    uint8_t *stage = static_cast<uint8_t *>(pinned_staging(p->ctx, probe_bytes + object_bytes + sizeof(double)));
+    double *l = reinterpret_cast<double *>(stage + probe_bytes + object_bytes);
+    check(cudaMemcpyAsync(stage, p->grad_p64.ptr, probe_bytes, cudaMemcpyDeviceToHost, s), "download gradient");
+    check(cudaMemcpyAsync(stage + probe_bytes, p->grad_o.ptr, object_bytes, cudaMemcpyDeviceToHost, s),
           "download gradient");
-    check(cudaStreamSynchronize(p->ctx->stream), "sync");
-    for (long long j = 0; j < p->objects; j++) {
-        if (re) re[j] = scale * (double)g[j].x;
-        if (im) im[j] = scale * (double)g[j].y;
-    }
+    check(cudaMemcpyAsync(l, p->loss_slot.ptr, sizeof(double), cudaMemcpyDeviceToHost, s), "loss");
+    check(cudaStreamSynchronize(s), "sync");
+    check_fault(p);
+    convert_out(reinterpret_cast<const C2<T> *>(stage + probe_bytes), (size_t)p->objects, scale, object);
+    convert_out(reinterpret_cast<const double2 *>(stage), (size_t)p->n, scale, probe);
+    if (loss) *loss = *l;
+}
+
+int backward(cubo_ptycho_plan *p, int recompute, double *loss, const ComplexOut &object, const ComplexOut &probe) {
+    if (!p) return CUBO_PTYCHO_INVALID_INPUT;
+    return run_guarded(p->ctx, [&] {
+        if (p->states > 1 || p->multislice) fail(CUBO_PTYCHO_UNSUPPORTED, "the adjoint pair is single-slice only");
+        if (recompute || !p->tape_valid) {
+            if (p->fp64) enqueue_forward<double>(p);
+            else enqueue_forward<float>(p);
+            p->tape_valid = true;
+        }
+        if (p->fp64) enqueue_gathers<double>(p);
+        else enqueue_gathers<float>(p);
+        // dL/dRe + i dL/dIm = -2 n * (sum of conj(.) dpsi): dpsi carries the inverse transform's 1/n
+        const double scale = -2.0 * (double)p->n;
+        if (p->fp64) download_gradients<double>(p, scale, object, probe, loss);
+        else download_gradients<float>(p, scale, object, probe, loss);
+    });
 }
 }  // namespace
 
@@ -2052,33 +2234,12 @@ int cubo_ptycho_plan_forward(cubo_ptycho_plan *p, double *loss) {
 
 int cubo_ptycho_plan_backward(cubo_ptycho_plan *p, int recompute, double *loss, double *gore, double *goim,
                               double *gpre, double *gpim) {
-    if (!p) return CUBO_PTYCHO_INVALID_INPUT;
-    return run_guarded(p->ctx, [&] {
-        if (p->states > 1 || p->multislice) fail(CUBO_PTYCHO_UNSUPPORTED, "the adjoint pair is single-slice only");
-        if (recompute || !p->tape_valid) {
-            if (p->fp64) enqueue_forward<double>(p);
-            else enqueue_forward<float>(p);
-            p->tape_valid = true;
-        }
-        if (p->fp64) enqueue_gathers<double>(p);
-        else enqueue_gathers<float>(p);
-        // dL/dRe + i dL/dIm = -2 n * (sum of conj(.) dpsi): dpsi carries the inverse transform's 1/n
-        const double scale = -2.0 * (double)p->n;
-        if (p->fp64) download_object_gradient<double>(p, scale, gore, goim);
-        else download_object_gradient<float>(p, scale, gore, goim);
-        std::vector<double2> gp(p->n);
-        double l = 0;
-        check(cudaMemcpyAsync(gp.data(), p->grad_p64.ptr, (size_t)p->n * sizeof(double2), cudaMemcpyDeviceToHost,
-                              p->ctx->stream), "download gradient");
-        check(cudaMemcpyAsync(&l, p->loss_slot.ptr, sizeof(double), cudaMemcpyDeviceToHost, p->ctx->stream), "loss");
-        check(cudaStreamSynchronize(p->ctx->stream), "sync");
-        check_fault(p);
-        for (int k = 0; k < p->n; k++) {
-            if (gpre) gpre[k] = scale * gp[k].x;
-            if (gpim) gpim[k] = scale * gp[k].y;
-        }
-        if (loss) *loss = l;
-    });
+    return backward(p, recompute, loss, ComplexOut{gore, goim, 1}, ComplexOut{gpre, gpim, 1});
+}
+
+int cubo_ptycho_plan_backward_complex(cubo_ptycho_plan *p, int recompute, double *loss, double *grad_object,
+                                      double *grad_probe) {
+    return backward(p, recompute, loss, interleaved(grad_object), interleaved(grad_probe));
 }
 
 int cubo_ptycho_plan_set_timing(cubo_ptycho_plan *p, int enabled) {
@@ -2351,6 +2512,16 @@ int cubo_ptycho_batch_get_state(cubo_ptycho_batch *b, int index, double *ore, do
 int cubo_ptycho_batch_errors(cubo_ptycho_batch *b, int index, int count, double *errors) {
     if (!b || index < 0 || index >= (int)b->plans.size()) return CUBO_PTYCHO_INVALID_INPUT;
     return cubo_ptycho_plan_errors(b->plans[index], count, errors);
+}
+
+int cubo_ptycho_batch_set_state_complex(cubo_ptycho_batch *b, int index, const double *object, const double *probe) {
+    if (!b || index < 0 || index >= (int)b->plans.size()) return CUBO_PTYCHO_INVALID_INPUT;
+    return cubo_ptycho_plan_set_state_complex(b->plans[index], object, probe);
+}
+
+int cubo_ptycho_batch_get_state_complex(cubo_ptycho_batch *b, int index, double *object, double *probe) {
+    if (!b || index < 0 || index >= (int)b->plans.size()) return CUBO_PTYCHO_INVALID_INPUT;
+    return cubo_ptycho_plan_get_state_complex(b->plans[index], object, probe);
 }
 
 long long cubo_ptycho_batch_launches_per_iteration(const cubo_ptycho_batch *b) {

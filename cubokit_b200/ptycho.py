@@ -140,6 +140,14 @@ def _split(z, shape=None):
     return re, im
 
 
+def _complex(z, shape=None):
+    """``z`` as contiguous interleaved complex128 values (``z`` itself where it is that already)."""
+    z = np.asarray(z)
+    if shape is not None and z.size != int(np.prod(shape)):
+        raise PtychographyError("array size")
+    return np.ascontiguousarray(z, dtype=np.complex128)
+
+
 def _ptr(a, t=C.c_double):
     return a.ctypes.data_as(C.POINTER(t))
 
@@ -295,15 +303,14 @@ class SingleslicePtychography:
             cb = L.PROGRESS_FN(_progress)
             inp.params.progress = cb
             inp.params.cancel = C.pointer(inp.cancel_flag)
-        ore, oim = _split(obj)
-        pre, pim = _split(prb)
+        obj_io = np.array(obj, dtype=np.complex128, order="C")
+        prb_io = np.array(prb, dtype=np.complex128, order="C")
         errors = np.zeros(max(int(iterations), 1))
-        st = ctx.lib.cubo_ptycho_reconstruct(ctx.handle, C.byref(inp.problem), C.byref(inp.params), _ptr(ore),
-                                             _ptr(oim), _ptr(pre), _ptr(pim), _ptr(errors))
+        st = ctx.lib.cubo_ptycho_reconstruct_complex(ctx.handle, C.byref(inp.problem), C.byref(inp.params),
+                                                     _ptr(obj_io), _ptr(prb_io), _ptr(errors))
         ctx.check(st)
         pos = np.column_stack(inp.positions_out) if inp.count else np.zeros((0, 2))
-        return Result((ore + 1j * oim).reshape(obj.shape), (pre + 1j * pim).reshape(prb.shape),
-                      errors[: int(iterations)].copy(), pos)
+        return Result(obj_io, prb_io, errors[: int(iterations)].copy(), pos)
 
 
 @dataclass
@@ -522,16 +529,13 @@ class Plan:
         self.handle = h
 
     def set_state(self, obj, probe):
-        ore, oim = _split(obj, self.object_shape)
-        pre, pim = _split(probe, self.probe_shape)
-        self.ctx.check(self.ctx.lib.cubo_ptycho_plan_set_state(self.handle, _ptr(ore), _ptr(oim), _ptr(pre), _ptr(pim)))
+        o, p = _complex(obj, self.object_shape), _complex(probe, self.probe_shape)
+        self.ctx.check(self.ctx.lib.cubo_ptycho_plan_set_state_complex(self.handle, _ptr(o), _ptr(p)))
 
     def get_state(self):
-        no = int(np.prod(self.object_shape))
-        npb = int(np.prod(self.probe_shape))
-        ore, oim, pre, pim = np.zeros(no), np.zeros(no), np.zeros(npb), np.zeros(npb)
-        self.ctx.check(self.ctx.lib.cubo_ptycho_plan_get_state(self.handle, _ptr(ore), _ptr(oim), _ptr(pre), _ptr(pim)))
-        return (ore + 1j * oim).reshape(self.object_shape), (pre + 1j * pim).reshape(self.probe_shape)
+        o, p = np.empty(self.object_shape, np.complex128), np.empty(self.probe_shape, np.complex128)
+        self.ctx.check(self.ctx.lib.cubo_ptycho_plan_get_state_complex(self.handle, _ptr(o), _ptr(p)))
+        return o, p
 
     def positions(self) -> np.ndarray:
         """The current scan positions (P, 2): the given ones, moved by position correction when it is on."""
@@ -595,15 +599,11 @@ class Plan:
 
     def backward(self, recompute_exit_waves: bool = False):
         """``(loss, grad_object, grad_probe)``: dL/dRe + i dL/dIm of the forward loss (``cubo_ptycho_plan_backward``)."""
-        no = int(np.prod(self.object_shape))
-        npb = int(np.prod(self.probe_shape))
-        gore, goim, gpre, gpim = np.zeros(no), np.zeros(no), np.zeros(npb), np.zeros(npb)
+        go, gp = np.empty(self.object_shape, np.complex128), np.empty(self.probe_shape, np.complex128)
         loss = C.c_double(0)
-        self.ctx.check(self.ctx.lib.cubo_ptycho_plan_backward(self.handle, 1 if recompute_exit_waves else 0,
-                                                              C.byref(loss), _ptr(gore), _ptr(goim), _ptr(gpre),
-                                                              _ptr(gpim)))
-        return (loss.value, (gore + 1j * goim).reshape(self.object_shape),
-                (gpre + 1j * gpim).reshape(self.probe_shape))
+        self.ctx.check(self.ctx.lib.cubo_ptycho_plan_backward_complex(self.handle, 1 if recompute_exit_waves else 0,
+                                                                      C.byref(loss), _ptr(go), _ptr(gp)))
+        return loss.value, go, gp
 
     def set_timing(self, enabled: bool):
         self.ctx.check(self.ctx.lib.cubo_ptycho_plan_set_timing(self.handle, 1 if enabled else 0))
@@ -675,18 +675,14 @@ class Batch:
 
     def set_state(self, index, obj, probe):
         os_, ps = self.shapes[index]
-        ore, oim = _split(obj, os_)
-        pre, pim = _split(probe, ps)
-        self.ctx.check(self.ctx.lib.cubo_ptycho_batch_set_state(self.handle, index, _ptr(ore), _ptr(oim), _ptr(pre),
-                                                                _ptr(pim)))
+        o, p = _complex(obj, os_), _complex(probe, ps)
+        self.ctx.check(self.ctx.lib.cubo_ptycho_batch_set_state_complex(self.handle, index, _ptr(o), _ptr(p)))
 
     def get_state(self, index):
         os_, ps = self.shapes[index]
-        no, npb = int(np.prod(os_)), int(np.prod(ps))
-        ore, oim, pre, pim = np.zeros(no), np.zeros(no), np.zeros(npb), np.zeros(npb)
-        self.ctx.check(self.ctx.lib.cubo_ptycho_batch_get_state(self.handle, index, _ptr(ore), _ptr(oim), _ptr(pre),
-                                                                _ptr(pim)))
-        return (ore + 1j * oim).reshape(os_), (pre + 1j * pim).reshape(ps)
+        o, p = np.empty(os_, np.complex128), np.empty(ps, np.complex128)
+        self.ctx.check(self.ctx.lib.cubo_ptycho_batch_get_state_complex(self.handle, index, _ptr(o), _ptr(p)))
+        return o, p
 
     def run(self, iterations: int, synchronize: bool = True):
         self.ctx.check(self.ctx.lib.cubo_ptycho_batch_run(self.handle, iterations, 1 if synchronize else 0))

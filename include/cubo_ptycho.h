@@ -162,6 +162,12 @@ CUBO_PTYCHO_API int cubo_ptycho_reconstruct(cubo_ptycho_context *context, const 
                             const cubo_ptycho_params *params, double *object_re, double *object_im, double *probe_re,
                             double *probe_im, double *errors);
 
+/* The same with complex arrays of interleaved (re, im) pairs, as C, C++, NumPy and Swift's Complex lay them out: no planes
+ * to split and join on the caller's side. */
+CUBO_PTYCHO_API int cubo_ptycho_reconstruct_complex(cubo_ptycho_context *context, const cubo_ptycho_problem *problem,
+                                                    const cubo_ptycho_params *params, double *object, double *probe,
+                                                    double *errors);
+
 /* ---- The mixed-state engine: MixedstatePtychography.reconstruct (PtychographyEngines.swift:121-262).  Several mutually
  * incoherent probe states share one object; the detector intensity is the sum of the states' far-field intensities.
  * Runs in the FP64 form (params->form must be CUBO_PTYCHO_FORM_FP64: the reference's engine is Double) with the shared
@@ -239,6 +245,10 @@ CUBO_PTYCHO_API int cubo_ptycho_plan_set_state(cubo_ptycho_plan *plan, const dou
                                const double *probe_re, const double *probe_im);
 CUBO_PTYCHO_API int cubo_ptycho_plan_get_state(cubo_ptycho_plan *plan, double *object_re, double *object_im, double *probe_re,
                                double *probe_im);
+/* The same with interleaved complex arrays. */
+CUBO_PTYCHO_API int cubo_ptycho_plan_set_state_complex(cubo_ptycho_plan *plan, const double *object,
+                                                       const double *probe);
+CUBO_PTYCHO_API int cubo_ptycho_plan_get_state_complex(cubo_ptycho_plan *plan, double *object, double *probe);
 /* The plan's current scan positions (count values each): the given ones, moved by position correction when it is on. */
 CUBO_PTYCHO_API int cubo_ptycho_plan_get_positions(cubo_ptycho_plan *plan, double *rows, double *columns);
 /* ---- Sharded iterations: one reconstruction's positions split into bands, one plan per band (per GPU), each holding
@@ -284,6 +294,10 @@ CUBO_PTYCHO_API int cubo_ptycho_plan_backward(cubo_ptycho_plan *plan, int recomp
                                               double *grad_object_re, double *grad_object_im, double *grad_probe_re,
                                               double *grad_probe_im);
 
+/* The same with interleaved complex gradients (either may be NULL). */
+CUBO_PTYCHO_API int cubo_ptycho_plan_backward_complex(cubo_ptycho_plan *plan, int recompute_exit_waves, double *loss,
+                                                      double *grad_object, double *grad_probe);
+
 /* ---- Batches: many independent reconstructions (each its own problem and parameters: scan, detector and object sizes
  * may differ) advanced together.  One iteration of every reconstruction of the batch is captured once into a CUDA graph
  * and replayed, so a run of the whole batch costs one graph launch per iteration.  No counterpart in the reference,
@@ -298,6 +312,11 @@ CUBO_PTYCHO_API int cubo_ptycho_batch_set_state(cubo_ptycho_batch *batch, int in
                                                 const double *probe_im);
 CUBO_PTYCHO_API int cubo_ptycho_batch_get_state(cubo_ptycho_batch *batch, int index, double *object_re,
                                                 double *object_im, double *probe_re, double *probe_im);
+/* The same with interleaved complex arrays. */
+CUBO_PTYCHO_API int cubo_ptycho_batch_set_state_complex(cubo_ptycho_batch *batch, int index, const double *object,
+                                                        const double *probe);
+CUBO_PTYCHO_API int cubo_ptycho_batch_get_state_complex(cubo_ptycho_batch *batch, int index, double *object,
+                                                        double *probe);
 /* Enqueues `iterations` replays of the captured iteration on the context stream; synchronize = 0 returns at once. */
 CUBO_PTYCHO_API int cubo_ptycho_batch_run(cubo_ptycho_batch *batch, int iterations, int synchronize);
 CUBO_PTYCHO_API int cubo_ptycho_batch_errors(cubo_ptycho_batch *batch, int index, int count, double *errors);
