@@ -180,15 +180,33 @@ template <typename T> int probe_gather_resident_ctas();  // CTAs of the probe ga
 template <typename T>
 cudaError_t launch_probe_reduce(const C2<T> *partial_grad, const T *partial_weight, int groups, int n,
                                 double2 *grad, double *weight, double *block_max, cudaStream_t s);
-cudaError_t launch_max_reduce(const double *values, int count, double *out, cudaStream_t s);
+int probe_reduce_blocks(int n);  // entries of block_max
+cudaError_t launch_maxima(const double *values, int arrays, long long stride, long long count, double *out,
+                          const double *last, long long last_count, double *out_last, cudaStream_t s);
 // The maximum of count values (float or double) into *out, one CTA in a fixed order.
 template <typename V> cudaError_t launch_max_values(const V *values, long long count, double *out, cudaStream_t s);
+// One iteration's updates: `slices` object slices of `objects` samples, each with its maximum weight object_max[slice], and
+// `states` probes of n samples (0: the probe stays).
 template <typename T>
-cudaError_t launch_object_update(C2<T> *object, const C2<T> *grad, const T *weight, int count, const double *max_weight,
-                                 double step, double minimum, int cap, int pure_phase, cudaStream_t s);
+struct UpdateArgs {
+    C2<T> *object;
+    const C2<T> *object_grad;
+    const T *object_weight;
+    int objects, slices;
+    const double *object_max;
+    double2 *probe;
+    const double2 *probe_grad;
+    const double *probe_weight;
+    int n, states;
+    const double *probe_max;
+    double step, minimum;
+    int cap, pure_phase;
+};
+template <typename T> cudaError_t launch_update(const UpdateArgs<T> &a, cudaStream_t s);
 // Fixed-order FP64 sum of error[0, count) divided by `divisor` into errors[*iteration], then ++*iteration.
 cudaError_t launch_error_reduce(const double *error, long long count, double divisor, double *errors, int *iteration,
                                 double *scratch, cudaStream_t s);
+int error_reduce_launches(long long count);
 int error_reduce_scratch();  // doubles of scratch launch_error_reduce needs
 // object-gather candidate lists on the device: without `list`, counts[tile * groups + group] = the number of the group's
 // positions whose window touches the tile; with it (and starts = exclusive sums of the counts), those positions in
@@ -341,8 +359,6 @@ cudaError_t launch_orthogonalize(double2 *probes, int states, int n, double2 *gr
 
 cudaError_t configure_fft_lines();
 cudaError_t launch_scale_f64(double2 *data, int count, double scale, cudaStream_t s);
-cudaError_t launch_probe_update(double2 *probe, const double2 *grad, const double *weight, int n, const double *max_weight,
-                                double step, double minimum, cudaStream_t s);
 // sums[0] = sum |p|^2, sums[1] = sum fr*R*w, sums[2] = sum fc*C*w (fixed order, one CTA)
 cudaError_t launch_probe_moments(const double2 *probe, int rows, int columns, double *sums, cudaStream_t s);
 cudaError_t launch_energy(const double2 *data, int n, double *sum, cudaStream_t s);

@@ -511,22 +511,39 @@ __global__ void __launch_bounds__(kProbeThreads) probe_gather_grouped_kernel(con
     probe_gather_body<T>(a, v % blocks, v / blocks);
 }
 
+// The groups' probe sums in FP64: 32 pixels a CTA, warp w takes the w-th eighth of the groups in order, then the eighths
+// are added in order.  (One thread a pixel over every group left 16 to 64 CTAs walking up to 148 partials: 62 us for 128 x
+// 128, 13 us now.)
+constexpr int kReducePixels = 32, kReduceSlices = 8;
 template <typename T>
 __global__ void __launch_bounds__(256) probe_reduce_kernel(const C2<T> *pg, const T *pw, int groups, int n,
                                                            double2 *grad, double *weight, double *block_max_out) {
-    __shared__ double scratch[32];
-    const int k = blockIdx.x * 256 + threadIdx.x;
+    __shared__ double sums[3][kReduceSlices][kReducePixels];
+    const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5, k = blockIdx.x * kReducePixels + lane;
     double gx = 0, gy = 0, w = 0;
     if (k < n) {
-        for (int g = 0; g < groups; g++) {
+        const int end = groups * (slice + 1) / kReduceSlices;
+        for (int g = groups * slice / kReduceSlices; g < end; g++) {
             const C2<T> v = pg[(size_t)g * n + k];
             gx += (double)v.x; gy += (double)v.y; w += (double)pw[(size_t)g * n + k];
         }
+    }
+    sums[0][slice][lane] = gx;
+    sums[1][slice][lane] = gy;
+    sums[2][slice][lane] = w;
+    __syncthreads();
+    if (slice > 0) return;
+    for (int q = 1; q < kReduceSlices; q++) {
+        gx += sums[0][q][lane];
+        gy += sums[1][q][lane];
+        w += sums[2][q][lane];
+    }
+    if (k < n) {
         grad[k] = make_double2(gx, gy);
         weight[k] = w;
     }
-    const double m = block_max<256>(k < n ? w : -DBL_MAX, scratch);
-    if (threadIdx.x == 0) block_max_out[blockIdx.x] = m;
+    const double m = warp_max(k < n ? w : -DBL_MAX);
+    if (lane == 0) block_max_out[blockIdx.x] = m;
 }
 
 template <typename V>
@@ -536,6 +553,21 @@ __global__ void __launch_bounds__(1024) max_reduce_kernel(const V *v, long long 
     for (long long i = threadIdx.x; i < count; i += 1024) m = fmax(m, (double)v[i]);
     m = block_max<1024>(m, scratch);
     if (threadIdx.x == 0) *out = m;
+}
+
+// The maximum of each of `arrays` arrays of `count` values, stride apart, into out[array], and of one more array into
+// *out_last: one CTA an array.
+__global__ void __launch_bounds__(1024) maxima_kernel(const double *v, int arrays, long long stride, long long count,
+                                                      double *out, const double *last, long long last_count,
+                                                      double *out_last) {
+    __shared__ double scratch[32];
+    const bool tail = (int)blockIdx.x == arrays;
+    const double *a = tail ? last : v + (size_t)blockIdx.x * stride;
+    const long long n = tail ? last_count : count;
+    double m = -DBL_MAX;
+    for (long long i = threadIdx.x; i < n; i += 1024) m = fmax(m, a[i]);
+    m = block_max<1024>(m, scratch);
+    if (threadIdx.x == 0) *(tail ? out_last : out + blockIdx.x) = m;
 }
 
 // Ptychography.swift:362-370,378-382: O += step / sqrt(1e-16 + ((1 - m) w)^2 + (m max w)^2) * grad, then the cap.
@@ -548,19 +580,33 @@ __device__ __forceinline__ void object_cap(C2<T> &o, int pure_phase) {
     else { o.x = target; o.y = 0; }
 }
 
+// The object's slices (blocks 0 .. object_blocks slices - 1, each slice with its own maximum weight) and the probe states
+// (the blocks after them, sharing one weight; Ptychography.swift:383-386): one launch for every sample an iteration updates.
 template <typename T>
-__global__ void __launch_bounds__(256) object_update_kernel(C2<T> *object, const C2<T> *grad, const T *weight,
-                                                            int count, const double *max_weight, double step,
-                                                            double minimum, int cap, int pure_phase) {
-    const int j = blockIdx.x * 256 + threadIdx.x;
-    if (j >= count) return;
-    const double l = (1 - minimum) * (double)weight[j], x = minimum * *max_weight;
-    const T s = (T)(step * (1 / sqrt(1e-16 + l * l + x * x)));
-    C2<T> o = object[j];
-    const C2<T> g = grad[j];
-    o.x += s * g.x; o.y += s * g.y;
-    if (cap || pure_phase) object_cap<T>(o, pure_phase);
-    object[j] = o;
+__global__ void __launch_bounds__(256) update_kernel(const __grid_constant__ UpdateArgs<T> a, int object_blocks) {
+    int block = blockIdx.x;
+    if (block < object_blocks * a.slices) {
+        const int slice = block / object_blocks, j = (block - slice * object_blocks) * 256 + threadIdx.x;
+        if (j >= a.objects) return;
+        const size_t i = (size_t)slice * a.objects + j;
+        const double l = (1 - a.minimum) * (double)a.object_weight[i], x = a.minimum * a.object_max[slice];
+        const T s = (T)(a.step * (1 / sqrt(1e-16 + l * l + x * x)));
+        C2<T> o = a.object[i];
+        const C2<T> g = a.object_grad[i];
+        o.x += s * g.x; o.y += s * g.y;
+        if (a.cap || a.pure_phase) object_cap<T>(o, a.pure_phase);
+        a.object[i] = o;
+        return;
+    }
+    block -= object_blocks * a.slices;
+    const int probe_blocks = (a.n + 255) / 256, state = block / probe_blocks;
+    const int k = (block - state * probe_blocks) * 256 + threadIdx.x;
+    if (k >= a.n) return;
+    const size_t i = (size_t)state * a.n + k;
+    const double l = (1 - a.minimum) * a.probe_weight[k], x = a.minimum * *a.probe_max;
+    const double s = a.step * (1 / sqrt(1e-16 + l * l + x * x));
+    a.probe[i].x += s * a.probe_grad[i].x;
+    a.probe[i].y += s * a.probe_grad[i].y;
 }
 
 // The cap alone, for position correction, which reads the updated object before it is capped (Ptychography.swift:371-381).
@@ -574,6 +620,7 @@ __global__ void __launch_bounds__(256) object_cap_kernel(C2<T> *object, int coun
 }
 
 constexpr int kErrorBlocks = 256;
+constexpr long long kErrorSingle = 32768;  // values one CTA sums in less time than a second launch takes
 
 // Stage 1: block b sums the fixed slice [b*count/B, (b+1)*count/B) (thread t takes every 1024th element of it, then a
 // fixed tree); stage 2 sums the B block sums in order.  No atomics: the same inputs give the same bits.
@@ -584,6 +631,20 @@ __global__ void __launch_bounds__(1024) error_partial_kernel(const double *error
     for (long long i = b + threadIdx.x; i < e; i += 1024) s += error[i];
     s = block_sum<1024>(s, scratch);
     if (threadIdx.x == 0) block_sums[blockIdx.x] = s;
+}
+
+// Up to kErrorSingle values in one launch: thread t takes every 1024th, then the fixed tree.
+__global__ void __launch_bounds__(1024) error_single_kernel(const double *error, int count, double divisor,
+                                                            double *errors, int *iteration) {
+    __shared__ double scratch[32];
+    double s = 0;
+    for (int i = threadIdx.x; i < count; i += 1024) s += error[i];
+    s = block_sum<1024>(s, scratch);
+    if (threadIdx.x == 0) {
+        const int it = *iteration;
+        errors[it] = s / divisor;
+        *iteration = it + 1;
+    }
 }
 
 __global__ void __launch_bounds__(kErrorBlocks) error_final_kernel(const double *block_sums, double divisor,
@@ -877,12 +938,15 @@ int probe_gather_resident_ctas() {
 template <typename T>
 cudaError_t launch_probe_reduce(const C2<T> *pg, const T *pw, int groups, int n, double2 *grad, double *weight,
                                 double *block_max_out, cudaStream_t s) {
-    probe_reduce_kernel<T><<<(n + 255) / 256, 256, 0, s>>>(pg, pw, groups, n, grad, weight, block_max_out);
+    probe_reduce_kernel<T><<<probe_reduce_blocks(n), 256, 0, s>>>(pg, pw, groups, n, grad, weight, block_max_out);
     return cudaGetLastError();
 }
 
-cudaError_t launch_max_reduce(const double *values, int count, double *out, cudaStream_t s) {
-    max_reduce_kernel<double><<<1, 1024, 0, s>>>(values, count, out);
+int probe_reduce_blocks(int n) { return (n + kReducePixels - 1) / kReducePixels; }
+
+cudaError_t launch_maxima(const double *values, int arrays, long long stride, long long count, double *out,
+                          const double *last, long long last_count, double *out_last, cudaStream_t s) {
+    maxima_kernel<<<arrays + 1, 1024, 0, s>>>(values, arrays, stride, count, out, last, last_count, out_last);
     return cudaGetLastError();
 }
 
@@ -895,10 +959,9 @@ template cudaError_t launch_max_values<float>(const float *, long long, double *
 template cudaError_t launch_max_values<double>(const double *, long long, double *, cudaStream_t);
 
 template <typename T>
-cudaError_t launch_object_update(C2<T> *object, const C2<T> *grad, const T *weight, int count, const double *max_weight,
-                                 double step, double minimum, int cap, int pure_phase, cudaStream_t s) {
-    object_update_kernel<T><<<(count + 255) / 256, 256, 0, s>>>(object, grad, weight, count, max_weight, step, minimum,
-                                                                 cap, pure_phase);
+cudaError_t launch_update(const UpdateArgs<T> &a, cudaStream_t s) {
+    const int object_blocks = (a.objects + 255) / 256, probe_blocks = (a.n + 255) / 256;
+    update_kernel<T><<<object_blocks * a.slices + probe_blocks * a.states, 256, 0, s>>>(a, object_blocks);
     return cudaGetLastError();
 }
 
@@ -909,6 +972,8 @@ cudaError_t launch_object_cap(C2<T> *object, int count, int pure_phase, cudaStre
 }
 
 int error_reduce_scratch() { return kErrorBlocks; }
+
+int error_reduce_launches(long long count) { return count <= kErrorSingle ? 1 : 2; }
 
 cudaError_t launch_tile_lists(const int *rr, const int *cc, int count, int rows, int columns, int object_rows,
                               int object_columns, int tile_w, int tile_h, int tiles_x, int tiles, int groups,
@@ -931,6 +996,10 @@ cudaError_t launch_amplitude_check(const float *amplitudes, long long count, dou
 
 cudaError_t launch_error_reduce(const double *error, long long count, double divisor, double *errors, int *iteration,
                                 double *scratch, cudaStream_t s) {
+    if (count <= kErrorSingle) {
+        error_single_kernel<<<1, 1024, 0, s>>>(error, (int)count, divisor, errors, iteration);
+        return cudaGetLastError();
+    }
     error_partial_kernel<<<kErrorBlocks, 1024, 0, s>>>(error, count, scratch);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -954,8 +1023,7 @@ cudaError_t launch_error_reduce(const double *error, long long count, double div
     template int probe_gather_resident_ctas<T>();                                                                      \
     template cudaError_t launch_probe_reduce<T>(const C2<T> *, const T *, int, int, double2 *, double *, double *,     \
                                                 cudaStream_t);                                                         \
-    template cudaError_t launch_object_update<T>(C2<T> *, const C2<T> *, const T *, int, const double *, double,       \
-                                                 double, int, int, cudaStream_t);                                      \
+    template cudaError_t launch_update<T>(const UpdateArgs<T> &, cudaStream_t);                                       \
     template cudaError_t launch_object_cap<T>(C2<T> *, int, int, cudaStream_t);
 INSTANTIATE(float)
 INSTANTIATE(double)

@@ -235,7 +235,7 @@ void parallel_ranges(size_t count, size_t grain, const F &body) {
     for (auto &t : threads) t.join();
 }
 
-constexpr size_t kConvertGrain = 1 << 16;  // values
+constexpr size_t kConvertGrain = 1 << 18;  // values: half a millisecond on one thread
 
 // The caller's complex arrays: a real and an imaginary plane (stride 1) or interleaved pairs (stride 2).
 struct ComplexIn {
@@ -288,54 +288,6 @@ void convert_out(const V *in, size_t count, double scale, const ComplexOut &out)
         if (out.im)
             for (size_t j = first; j < last; j++) out.im[j] = scale * (double)in[j].y;
     });
-}
-
-// Copies `bytes` of host memory to the device.  Page-locked memory goes as it is; pageable memory of some size through
-// page-locked pieces that several threads fill while earlier ones travel (the driver's own staging is one thread: 9.4 MB of
-// amplitudes took 1.2 ms, this way 0.4).
-void upload_host(cubo_ptycho_context *ctx, void *dst, const void *src, size_t bytes) {
-    constexpr size_t kPiece = 1 << 20, kLeast = 4 << 20, kThreads = 8;
-    cudaPointerAttributes at{};
-    const bool known = cudaPointerGetAttributes(&at, src) == cudaSuccess;
-    if (!known) (void)cudaGetLastError();
-    if (bytes < kLeast || (known && at.type != cudaMemoryTypeUnregistered)) {
-        check(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream), "upload");
-        return;
-    }
-    // two pieces per thread; the staging buffer may still feed earlier copies of this stream
-    check(cudaStreamSynchronize(ctx->stream), "sync");
-    uint8_t *stage = static_cast<uint8_t *>(pinned_staging(ctx, 2 * kThreads * kPiece));
-    cudaEvent_t events[2 * kThreads] = {};
-    cudaError_t failed = cudaSuccess;
-    for (auto &e : events)
-        if (failed == cudaSuccess) failed = cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
-    const size_t pieces = (bytes + kPiece - 1) / kPiece;
-    std::atomic<size_t> next{0};
-    std::atomic<int> error{(int)failed};
-    if (failed == cudaSuccess)
-        parallel_ranges(kThreads, 1, [&](size_t first, size_t last) {
-            cudaError_t e = cudaSetDevice(ctx->device);
-            for (size_t turn = 0; e == cudaSuccess && error == 0; turn++) {
-                const size_t piece = next++;
-                if (piece >= pieces) break;
-                // ranges are one slot pair each, or several where fewer threads run
-                const size_t slot = 2 * first + turn % (2 * (last - first));
-                uint8_t *at_piece = stage + slot * kPiece;
-                const size_t off = piece * kPiece, size = std::min(kPiece, bytes - off);
-                if (turn >= 2 * (last - first)) e = cudaEventSynchronize(events[slot]);
-                std::memcpy(at_piece, static_cast<const uint8_t *>(src) + off, size);
-                if (e == cudaSuccess)
-                    e = cudaMemcpyAsync(static_cast<uint8_t *>(dst) + off, at_piece, size, cudaMemcpyHostToDevice,
-                                        ctx->stream);
-                if (e == cudaSuccess) e = cudaEventRecord(events[slot], ctx->stream);
-            }
-            if (e != cudaSuccess) error = (int)e;
-        });
-    const cudaError_t done = cudaStreamSynchronize(ctx->stream);  // the pieces are free again
-    for (auto &e : events)
-        if (e) cudaEventDestroy(e);
-    check((cudaError_t)error.load(), "upload");
-    check(done, "upload");
 }
 
 }  // namespace
@@ -705,10 +657,9 @@ void build_plan(cubo_ptycho_plan *p, const cubo_ptycho_problem *pr) {
     build_scan(p, pr->position_rows, pr->position_columns);
     // ---- amplitudes (Float32, [position][row][column]; the 128 x 128 kernel's register order when it runs)
     check(p->amplitudes.alloc((size_t)P * n * sizeof(float)), "cudaMalloc amplitudes");
-    if (pr->amplitudes_on_device)
-        check(cudaMemcpyAsync(p->amplitudes.ptr, pr->amplitudes, (size_t)P * n * sizeof(float), cudaMemcpyDeviceToDevice, s),
-              "copy amplitudes");
-    else upload_host(p->ctx, p->amplitudes.ptr, pr->amplitudes, (size_t)P * n * sizeof(float));
+    check(cudaMemcpyAsync(p->amplitudes.ptr, pr->amplitudes, (size_t)P * n * sizeof(float),
+                          pr->amplitudes_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s),
+          "upload amplitudes");
     {
         // every amplitude finite and non-negative, and sum A^2 (Ptychography.swift:247-259), in the supplied order
         DeviceBuffer scratch, bad;
@@ -813,8 +764,8 @@ void build_plan(cubo_ptycho_plan *p, const cubo_ptycho_problem *pr) {
     check(p->partial_weight.alloc((size_t)p->groups * n * sizeof(T)), "cudaMalloc");
     check(p->grad_p64.alloc((size_t)p->states * n * sizeof(double2)), "cudaMalloc");
     check(p->weight_p64.alloc((size_t)n * sizeof(double)), "cudaMalloc");
-    p->probe_blocks = kblocks;
-    check(p->probe_block_max.alloc((size_t)kblocks * sizeof(double)), "cudaMalloc");
+    p->probe_blocks = probe_reduce_blocks(n);
+    check(p->probe_block_max.alloc((size_t)p->probe_blocks * sizeof(double)), "cudaMalloc");
     check(p->maxes.alloc(4 * sizeof(double)), "cudaMalloc");
     check(p->error_scratch.alloc((size_t)error_reduce_scratch() * sizeof(double)), "cudaMalloc");
     check(p->loss_slot.alloc(2 * sizeof(double)), "cudaMalloc");  // [0] the loss, [1] an int counter
@@ -936,8 +887,22 @@ void enqueue_shift_table(cubo_ptycho_plan *p) {
     for (int st = 0; st < p->states; st++) enqueue_shift_table_state<T>(p, st);
 }
 
-// Probe update and constraints, FP64 (Ptychography.swift:383-395).  With several probe states
-// (PtychographyEngines.swift:212-244): every state takes its own gradient with the shared normalisation; the centre of
+// The object update's and (the probe not fixed) the probe update's arguments: one slice, the object uncapped.  With several
+// probe states (PtychographyEngines.swift:212-244) every state takes its own gradient with the shared normalisation.
+// Position correction, which follows the object update, reads the shift table of the iteration, not the probe.
+template <typename T>
+UpdateArgs<T> update_args(const cubo_ptycho_plan *p) {
+    UpdateArgs<T> u{};
+    u.object = p->object.as<C2<T>>(); u.object_grad = p->grad_o.as<C2<T>>(); u.object_weight = p->weight_o.as<T>();
+    u.objects = (int)p->objects; u.slices = 1; u.object_max = p->maxes.as<double>();
+    u.probe = p->probe64.as<double2>(); u.probe_grad = p->grad_p64.as<double2>();
+    u.probe_weight = p->weight_p64.as<double>(); u.n = p->n; u.states = p->params.fix_probe ? 0 : p->states;
+    u.probe_max = p->maxes.as<double>() + 1;
+    u.step = p->params.step_size; u.minimum = p->params.normalization_minimum;
+    return u;
+}
+
+// Probe constraints after its update, FP64 (Ptychography.swift:386-395).  With several probe states the centre of
 // mass of state 0 shifts every state; the aperture constrains state 0; the amplitude constraint and the support apply
 // to every state; then the orthogonalisation.
 void enqueue_probe_side(cubo_ptycho_plan *p) {
@@ -947,12 +912,6 @@ void enqueue_probe_side(cubo_ptycho_plan *p) {
     double2 *probes = p->probe64.as<double2>(), *x = p->scratch64.as<double2>();
     double *sums = p->sums.as<double>();
     if (!pp.fix_probe) {
-        for (int st = 0; st < S; st++)
-            timed(p, kProbeSide, 1, [&] {
-                return launch_probe_update(probes + (size_t)st * n, p->grad_p64.as<double2>() + (size_t)st * n,
-                                           p->weight_p64.as<double>(), n, p->maxes.as<double>() + 1, pp.step_size,
-                                           pp.normalization_minimum, s);
-            });
         if (pp.fix_probe_center_of_mass) {  // PtychographyConstraints.swift:34-37: the centre of mass of state 0
             timed(p, kProbeSide, 1, [&] { return launch_probe_moments(probes, p->R, p->C, sums, s); });
             for (int st = 0; st < S; st++) {
@@ -1160,10 +1119,9 @@ void enqueue_gathers(cubo_ptycho_plan *p) {
                                           p->probe_block_max.as<double>(), s);
         });
     }
-    timed(p, kMaxReduce, 2, [&] {
-        cudaError_t e = launch_max_reduce(p->tile_max.as<double>(), p->gather_maxima, p->maxes.as<double>(), s);
-        if (e == cudaSuccess) e = launch_max_reduce(p->probe_block_max.as<double>(), p->probe_blocks, p->maxes.as<double>() + 1, s);
-        return e;
+    timed(p, kMaxReduce, 1, [&] {
+        return launch_maxima(p->tile_max.as<double>(), 1, 0, p->gather_maxima, p->maxes.as<double>(),
+                             p->probe_block_max.as<double>(), p->probe_blocks, p->maxes.as<double>() + 1, s);
     });
 }
 
@@ -1224,10 +1182,9 @@ void enqueue_banded_pass_and_gathers(cubo_ptycho_plan *p) {
                                           p->grad_p64.as<double2>(), p->weight_p64.as<double>(),
                                           p->probe_block_max.as<double>(), s);
     });
-    timed(p, kMaxReduce, 2, [&] {
-        cudaError_t e = launch_max_reduce(p->tile_max.as<double>(), p->gather_maxima, p->maxes.as<double>(), s);
-        if (e == cudaSuccess) e = launch_max_reduce(p->probe_block_max.as<double>(), p->probe_blocks, p->maxes.as<double>() + 1, s);
-        return e;
+    timed(p, kMaxReduce, 1, [&] {
+        return launch_maxima(p->tile_max.as<double>(), 1, 0, p->gather_maxima, p->maxes.as<double>(),
+                             p->probe_block_max.as<double>(), p->probe_blocks, p->maxes.as<double>() + 1, s);
     });
 }
 
@@ -1286,9 +1243,10 @@ void enqueue_iteration_tail(cubo_ptycho_plan *p) {
     const bool threshold = p->states > 1 || pp.constrain_object_amplitude;
     const int cap = !correct && threshold ? 1 : 0, pure = !correct && pp.pure_phase_object ? 1 : 0;
     timed(p, kObjectUpdate, 1, [&] {
-        return launch_object_update<T>(p->object.as<C2<T>>(), p->grad_o.as<C2<T>>(), p->weight_o.as<T>(),
-                                       (int)p->objects, p->maxes.as<double>(), pp.step_size, pp.normalization_minimum,
-                                       cap, pure, s);
+        UpdateArgs<T> u = update_args<T>(p);
+        u.cap = cap;
+        u.pure_phase = pure;
+        return launch_update<T>(u, s);
     });
     if (correct) {
         enqueue_position_correction(p);
@@ -1304,7 +1262,7 @@ void enqueue_iteration_tail(cubo_ptycho_plan *p) {
             return launch_position_center(p->positions64.as<double>(), p->P, p->initial_mean_row,
                                           p->initial_mean_column, s);
         });
-    timed(p, kErrorReduce, 2, [&] {
+    timed(p, kErrorReduce, error_reduce_launches(p->error_count), [&] {
         return launch_error_reduce(p->error.as<double>(), p->error_count, p->divisor, p->errors.as<double>(),
                                    p->iteration.as<int>(), p->error_scratch.as<double>(), s);
     });
@@ -1415,32 +1373,27 @@ void enqueue_multislice_iteration(cubo_ptycho_plan *p) {
         return launch_probe_reduce<double>(pg.partial_grad, pg.partial_weight, p->groups, n, p->grad_p64.as<double2>(),
                                            p->weight_p64.as<double>(), p->probe_block_max.as<double>(), s);
     });
-    timed(p, kMaxReduce, L + 1, [&] {
-        cudaError_t e = cudaSuccess;
-        for (int sl = 0; sl < L && e == cudaSuccess; sl++)
-            e = launch_max_reduce(p->tile_max.as<double>() + (size_t)sl * p->gather_maxima, p->gather_maxima,
-                                  p->slice_max.as<double>() + sl, s);
-        if (e == cudaSuccess)
-            e = launch_max_reduce(p->probe_block_max.as<double>(), p->probe_blocks, p->maxes.as<double>() + 1, s);
-        return e;
+    timed(p, kMaxReduce, 1, [&] {
+        return launch_maxima(p->tile_max.as<double>(), L, p->gather_maxima, p->gather_maxima, p->slice_max.as<double>(),
+                             p->probe_block_max.as<double>(), p->probe_blocks, p->maxes.as<double>() + 1, s);
     });
     // updates (:547-572): each slice with its own maximum weight; identical slices averaged before the threshold,
     // which always applies
     const bool identical = p->identical_slices;
-    timed(p, kObjectUpdate, L + (identical ? 2 : 0), [&] {
-        cudaError_t e = cudaSuccess;
-        for (int sl = 0; sl < L && e == cudaSuccess; sl++)
-            e = launch_object_update<double>(obj + (size_t)sl * plane, p->grad_o.as<double2>() + (size_t)sl * plane,
-                                             p->weight_o.as<double>() + (size_t)sl * plane, (int)plane,
-                                             p->slice_max.as<double>() + sl, pp.step_size, pp.normalization_minimum,
-                                             identical ? 0 : 1, !identical && pp.pure_phase_object ? 1 : 0, s);
+    timed(p, kObjectUpdate, 1 + (identical ? 2 : 0), [&] {
+        UpdateArgs<double> u = update_args<double>(p);
+        u.slices = L;
+        u.object_max = p->slice_max.as<double>();
+        u.cap = identical ? 0 : 1;
+        u.pure_phase = !identical && pp.pure_phase_object ? 1 : 0;
+        cudaError_t e = launch_update<double>(u, s);
         if (identical && e == cudaSuccess) e = launch_average_slices(obj, L, plane, s);
         if (identical && e == cudaSuccess)
             e = launch_object_cap<double>(obj, (int)(L * plane), pp.pure_phase_object ? 1 : 0, s);
         return e;
     });
     enqueue_probe_side(p);
-    timed(p, kErrorReduce, 2, [&] {
+    timed(p, kErrorReduce, error_reduce_launches(p->error_count), [&] {
         return launch_error_reduce(p->error.as<double>(), p->error_count, p->divisor, p->errors.as<double>(),
                                    p->iteration.as<int>(), p->error_scratch.as<double>(), s);
     });
@@ -1455,7 +1408,7 @@ void enqueue_shard_gradients(cubo_ptycho_plan *p) {
     enqueue_position_pass<T>(p);
     enqueue_gathers<T>(p);
     check(cudaMemsetAsync(p->shard_counter.ptr, 0, sizeof(int), s), "memset");
-    timed(p, kErrorReduce, 2, [&] {
+    timed(p, kErrorReduce, error_reduce_launches(p->error_count), [&] {
         return launch_error_reduce(p->error.as<double>(), p->error_count, 1.0, p->shard_loss.as<double>(),
                                    p->shard_counter.as<int>(), p->error_scratch.as<double>(), s);
     });
@@ -1474,9 +1427,10 @@ void enqueue_shard_update(cubo_ptycho_plan *p) {
     });
     const bool threshold = p->states > 1 || pp.constrain_object_amplitude;
     timed(p, kObjectUpdate, 1, [&] {
-        return launch_object_update<T>(p->object.as<C2<T>>(), p->grad_o.as<C2<T>>(), p->weight_o.as<T>(),
-                                       (int)p->objects, p->maxes.as<double>(), pp.step_size, pp.normalization_minimum,
-                                       threshold ? 1 : 0, pp.pure_phase_object ? 1 : 0, s);
+        UpdateArgs<T> u = update_args<T>(p);
+        u.cap = threshold ? 1 : 0;
+        u.pure_phase = pp.pure_phase_object ? 1 : 0;
+        return launch_update<T>(u, s);
     });
     enqueue_probe_side(p);
 }
@@ -2170,7 +2124,7 @@ void enqueue_forward(cubo_ptycho_plan *p) {
     refresh_scan(p);
     enqueue_position_pass<T>(p);
     check(cudaMemsetAsync(p->loss_slot.ptr, 0, 2 * sizeof(double), p->ctx->stream), "memset");
-    timed(p, kErrorReduce, 2, [&] {
+    timed(p, kErrorReduce, error_reduce_launches(p->error_count), [&] {
         return launch_error_reduce(p->error.as<double>(), p->error_count, 1.0, p->loss_slot.as<double>(),
                                    reinterpret_cast<int *>(p->loss_slot.as<double>() + 1), p->error_scratch.as<double>(),
                                    p->ctx->stream);
@@ -2300,9 +2254,20 @@ struct cubo_ptycho_batch {
     // 64.2 ms per iteration against 57.8 ms in one wave and 61.3 ms with every item launching its own kernels.
     size_t wave_bytes = SIZE_MAX;
     std::vector<int> wave_of;  // per plan
+    // The items' own launches (shifted probes, passes that are not grouped, reductions, updates, constraints) are captured
+    // on these streams in turn, so that the graph runs them side by side: in one chain the small launches of twelve items
+    // took a tenth of the iteration.
+    static constexpr int kBranches = 8;
+    cudaStream_t branches[kBranches] = {};
+    cudaEvent_t fork = nullptr, joins[kBranches] = {};
     ~cubo_ptycho_batch() {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
+        if (fork) cudaEventDestroy(fork);
+        for (auto e : joins)
+            if (e) cudaEventDestroy(e);
+        for (auto b : branches)
+            if (b) cudaStreamDestroy(b);
         for (auto *p : plans) delete p;
     }
 };
@@ -2400,6 +2365,33 @@ cudaError_t launch_group(const cubo_ptycho_batch::Group &g, cudaStream_t s) {
     return launch_probe_gather_grouped<T>(g.args.as<ProbeGatherArgs<T>>(), g.offsets.as<int>(), items, total, s);
 }
 
+// body(plan) for every item of wave w, captured on the batch's branch streams: each branch follows what the context's
+// stream holds, and that stream follows every branch.
+template <typename F>
+void captured_branches(cubo_ptycho_batch *b, int w, const F &body) {
+    struct Restore {  // the enqueue functions take their stream from the context
+        cubo_ptycho_context *ctx;
+        cudaStream_t stream;
+        ~Restore() { ctx->stream = stream; }
+    } restore{b->ctx, b->ctx->stream};
+    check(cudaEventRecord(b->fork, restore.stream), "fork");
+    int used = 0, turn = 0;
+    for (size_t i = 0; i < b->plans.size(); i++) {
+        if (b->wave_of[i] != w) continue;
+        const int k = turn++ % cubo_ptycho_batch::kBranches;
+        if (k == used) {
+            check(cudaStreamWaitEvent(b->branches[k], b->fork, 0), "fork");
+            used++;
+        }
+        b->ctx->stream = b->branches[k];
+        body(b->plans[i]);
+    }
+    for (int k = 0; k < used; k++) {
+        check(cudaEventRecord(b->joins[k], b->branches[k]), "join");
+        check(cudaStreamWaitEvent(restore.stream, b->joins[k], 0), "join");
+    }
+}
+
 // Captures one iteration of every plan of the batch into a graph (again when an error buffer moved), wave by wave: the
 // wave's shifted probes and own position passes, its grouped passes, its grouped gathers, then its items' own gathers,
 // reductions, updates, constraints and error.
@@ -2409,26 +2401,27 @@ void capture_batch(cubo_ptycho_batch *b) {
     cudaStream_t s = b->ctx->stream;
     build_groups(b);
     check(cudaStreamSynchronize(s), "batch groups");
+    if (!b->fork) check(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming), "event");
+    for (int k = 0; k < cubo_ptycho_batch::kBranches; k++) {
+        if (!b->branches[k]) check(cudaStreamCreateWithFlags(&b->branches[k], cudaStreamNonBlocking), "stream");
+        if (!b->joins[k]) check(cudaEventCreateWithFlags(&b->joins[k], cudaEventDisableTiming), "event");
+    }
     long long before = 0;
     for (auto *p : b->plans) before += p->launches;
     check(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
     try {
         const int waves = b->plans.empty() ? 0 : b->wave_of.back() + 1;
         for (int w = 0; w < waves; w++) {
-            for (size_t i = 0; i < b->plans.size(); i++) {
-                if (b->wave_of[i] != w) continue;
-                cubo_ptycho_plan *p = b->plans[i];
+            captured_branches(b, w, [](cubo_ptycho_plan *p) {
                 if (p->banded) enqueue_banded_pass_and_gathers(p);
                 else if (p->fp64) enqueue_position_pass<double>(p);
                 else enqueue_position_pass<float>(p);
-            }
+            });
             for (int kind = 0; kind < 4; kind++)  // the wave's passes before any of its gathers
                 for (const auto &g : b->groups)
                     if (g->wave == w && g->kind == kind)
                         check(g->fp64 ? launch_group<double>(*g, s) : launch_group<float>(*g, s), "grouped launch");
-            for (size_t i = 0; i < b->plans.size(); i++) {
-                if (b->wave_of[i] != w) continue;
-                cubo_ptycho_plan *p = b->plans[i];
+            captured_branches(b, w, [](cubo_ptycho_plan *p) {
                 if (p->fp64) {
                     if (!p->banded) enqueue_gathers<double>(p);
                     enqueue_iteration_tail<double>(p);
@@ -2436,7 +2429,7 @@ void capture_batch(cubo_ptycho_batch *b) {
                     if (!p->banded) enqueue_gathers<float>(p);
                     enqueue_iteration_tail<float>(p);
                 }
-            }
+            });
         }
     } catch (...) {
         cudaGraph_t g = nullptr;

@@ -99,17 +99,6 @@ __global__ void scale_kernel(double2 *d, int count, double s) {
     if (i < count) { d[i].x *= s; d[i].y *= s; }
 }
 
-// Ptychography.swift:383-386
-__global__ void probe_update_kernel(double2 *probe, const double2 *grad, const double *weight, int n,
-                                    const double *max_weight, double step, double minimum) {
-    const int k = blockIdx.x * 256 + threadIdx.x;
-    if (k >= n) return;
-    const double l = (1 - minimum) * weight[k], x = minimum * *max_weight;
-    const double s = step * (1 / sqrt(1e-16 + l * l + x * x));
-    probe[k].x += s * grad[k].x;
-    probe[k].y += s * grad[k].y;
-}
-
 // PtychographyConstraints.swift:9-18: total intensity and its corner-centred first moments.
 __global__ void __launch_bounds__(1024) moments_kernel(const double2 *p, int rows, int columns, double *sums) {
     __shared__ double scratch[32];
@@ -299,12 +288,6 @@ cudaError_t configure_fft_lines() {
 
 cudaError_t launch_scale_f64(double2 *data, int count, double scale, cudaStream_t s) {
     scale_kernel<<<blocks(count), 256, 0, s>>>(data, count, scale);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_probe_update(double2 *probe, const double2 *grad, const double *weight, int n,
-                                const double *max_weight, double step, double minimum, cudaStream_t s) {
-    probe_update_kernel<<<blocks(n), 256, 0, s>>>(probe, grad, weight, n, max_weight, step, minimum);
     return cudaGetLastError();
 }
 

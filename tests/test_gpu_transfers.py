@@ -1,5 +1,5 @@
-"""Host arrays to and from the device: large pageable amplitudes (staged in pieces by several threads), and the
-interleaved complex calls beside the ones with a real and an imaginary plane."""
+"""Host arrays to and from the device: pageable, page-locked and device amplitudes, and the interleaved complex calls
+beside the ones with a real and an imaginary plane."""
 import ctypes as C
 
 import numpy as np
@@ -11,12 +11,12 @@ pytestmark = pytest.mark.gpu
 
 
 def _scene():
-    # 300 x 290 object pixels (more than one thread's range of values), 9.2 MB of amplitudes whose last piece is ragged
+    # 840 x 790 object pixels: two ranges of values, converted by two threads
     rng = np.random.default_rng(3)
     probe = scenes.raster_scene(scan=2, det=40, step=4, seed=5)["probe"]
-    positions = np.stack([rng.integers(20, 280, 1437), rng.integers(20, 270, 1437)], 1).astype(np.float64)
+    positions = np.stack([rng.integers(20, 820, 1437), rng.integers(20, 770, 1437)], 1).astype(np.float64)
     amplitudes = rng.uniform(0, 2, (1437, 40, 40)).astype(np.float32)
-    obj = np.exp(1j * rng.normal(0, 0.1, (300, 290)))
+    obj = np.exp(1j * rng.normal(0, 0.1, (840, 790)))
     return amplitudes, positions, obj, probe
 
 
