@@ -281,53 +281,48 @@ cudaError_t launch_spectrum_multiply(double2 *data, long long planes, int n, con
 // identicalSlices: every slice becomes the mean of the slices.
 cudaError_t launch_average_slices(double2 *object, int slices, long long plane, cudaStream_t s);
 
-// plane128.cu: the 128 x 128 FP64 plane transform of positions first .. first + count - 1 in one launch, one cluster
-// of plane128_cluster() CTAs per plane.  kPlaneFull: the input plane (times the object patch) -> FFT -> the pointwise
-// step -> inverse FFT (unscaled) -> out; kPlaneForward: the input (times the patch) -> FFT -> out, unscaled;
-// kPlaneInverse: a spectrum -> the pointwise step -> inverse FFT (unscaled) -> out.
-enum { kPlaneFull = 0, kPlaneForward = 1, kPlaneInverse = 2 };
-enum { kInputByPosition = 0, kInputByClass = 1 };
-enum { kPointwiseNone = 0, kPointwiseFactors = 1, kPointwiseProjection = 2, kPointwiseSolve = 3,
-       kPointwiseFactorPlane = 4 };
-struct Plane128Args {
-    int mode;
-    int first, count;
-    const double2 *in;              // input plane of position p: in + (p, scan.cls[p] by in_kind) * 16384
-    int in_kind;
-    const double2 *object;          // full / forward: the object patch factor, conjugated when conj_object; null: none
-    int conj_object;
-    int object_row_offset, object_column_offset;  // the patch one row / column further (position correction)
+// rowcol64.cu: FP64 planes as row and column launches through global memory (sides above 16 without a prime factor above
+// 13).  Every call covers positions [first, first + count).
+struct RcGeometry {
+    int rows, columns, object_rows, object_columns;
     ScanTables scan;
-    int object_rows, object_columns;
-    int pointwise;                  // kPointwiseFactors: x prop_rows[kr] prop_columns[kc] x scale; kPointwiseProjection
-                                    // (full mode): modulus projection with amplitudes (x inv_n) and error[p]
-    const double2 *prop_rows;       // 128 factors of the row frequency
-    const double2 *prop_columns;    // 128 of the column frequency; both conjugated when conj_prop
-    int conj_prop;
-    double scale;
-    const float *amplitudes;        // [positions][128 x 128]
-    double *error;                  // [positions] squared amplitude residual
-    double inv_n;
-    const double2 *tw;              // W_128^k, k = 0..127 (forward sign)
-    double2 *out;                   // output plane of position p: out + (p * out_stride + out_offset) * 16384
-    long long out_stride, out_offset;
-    int *fault;                     // set when a bulk copy's wait ran out
-    int ahead;                      // L2 prefetch distance in planes (0: the clusters resident at once)
-    // forward mode with kPointwiseSolve (position correction): the spectrum is the far field of the updated object one
-    // column further; with the forward model's far field and the one of the updated object one row further
-    // (far + ((p - first) * 2 + 0 or 1) * 16384) and the amplitudes, position p's 2 x 2 normal equations are summed and
-    // the position moved (positions / initial [rows | columns] of position_count); nothing is written to out
-    const double2 *far;
-    double *positions;
-    const double *initial;
-    int position_count;
-    double position_step_size, limit_update, limit_total;
-    int *position_bad;
-    const double *factors;          // inverse mode with kPointwiseFactorPlane: [positions][128 x 128] real scales
+    const double2 *tw_rows, *tw_columns;  // W_rows^t, W_columns^t
 };
-int plane128_cluster();
-cudaError_t configure_plane128();
-cudaError_t launch_plane128(const Plane128Args &a, int cluster, cudaStream_t s);
+// Row transforms of `layers` planes a position.  Forward: in (+ layer in_layer + (scan.cls[p] when by_class, else p)
+// planes) times the object patch (object null: no factor; conjugated when conj_object; object_after non-null: layer 0 has
+// `object` at the centre, layers 1 and 2 object_after a row and a column further) into out + layer out_layer +
+// (p - out_first) out_stride.  Inverse: in place in out.
+struct RcRows {
+    const double2 *in;
+    int by_class;
+    long long in_layer;
+    const double2 *object, *object_after;
+    int conj_object;
+    double2 *out;
+    long long out_layer, out_stride;
+    int out_first, first, count, layers;
+};
+// Columns, in place in planes + layer `layer` + (p - plane_first) stride: with `terms` the normal equations of position
+// correction from three layers ([p - plane_first][rowcol64_parts][5], nothing written back), with prop_rows the separable
+// propagator (conjugated when conj_prop) over n, else the projection (summed over the layers' intensities when there are
+// several) with its squared error per part, error[p rowcol64_parts + part].
+struct RcColumns {
+    double2 *planes;
+    long long layer, stride;
+    int plane_first, first, count, layers;
+    const float *amplitudes;
+    double *error;
+    const double2 *prop_rows, *prop_columns;
+    int conj_prop, zero_infinite;
+    double *terms;
+};
+bool rowcol64_applicable(int rows, int columns, int layers);
+int rowcol64_parts(int rows, int columns, int layers);  // column CTAs of a position
+cudaError_t configure_rowcol64();
+cudaError_t launch_rc_rows(const RcGeometry &q, const RcRows &r, bool inverse, cudaStream_t s);
+cudaError_t launch_rc_columns(const RcGeometry &q, const RcColumns &c, cudaStream_t s);
+cudaError_t launch_rc_move(const double *terms, int per, int first, int m, double *positions, const double *initial,
+                           int count, double step, double limit_update, double limit_total, int *bad, cudaStream_t s);
 
 // peaks.cu: the FP32 and FP64 FMA rates of the device (TFLOP/s, best of three timed launches on stream s).
 cudaError_t measure_fma_peaks(cudaStream_t s, int sms, double *fp32_tflops, double *fp64_tflops);
@@ -347,11 +342,6 @@ struct MixedPassArgs {
 };
 // Exit waves of every state, their far fields, the summed-intensity projection, the inverse transforms.
 cudaError_t launch_mixed_position_pass(const MixedPassArgs &a, const Fft2Plan64 &fft, int *launches, cudaStream_t s);
-// The summed-intensity projection's common factor of every pixel of the states' far fields dpsi[state][position][pixel]
-// into factors[position][pixel] (the inverse transform's 1/n folded in), the states left as they are, the per-position
-// error written.
-cudaError_t launch_mixed_factors(const double2 *dpsi, const float *amplitudes, int count, int states, int n,
-                                 bool zero_pixel_infinite, double *error, double *factors, cudaStream_t s);
 // The states become the eigenvectors of their Gram matrix, by decreasing intensity (gram, mixing: states^2 values;
 // scratch: states * n).
 cudaError_t launch_orthogonalize(double2 *probes, int states, int n, double2 *gram, double2 *mixing, double2 *scratch,

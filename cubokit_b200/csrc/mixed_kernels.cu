@@ -55,12 +55,10 @@ __device__ double block_sum_project(double v, double *scratch) {
     return s;
 }
 
-// With `factors` the common factor of each pixel is written there and the states are left as they are (the inverse
-// plane launches apply it); without, the states are scaled in place.
+// The summed-intensity projection: the states of position p are scaled by the common factor of each pixel.
 __global__ void __launch_bounds__(kProjectThreads) mixed_project_kernel(double2 *dpsi, const float *amplitudes, int first,
                                                                         int count, int states, int n, double inv_n,
-                                                                        int zero_infinite, double *error,
-                                                                        double *factors) {
+                                                                        int zero_infinite, double *error) {
     __shared__ double scratch[kProjectThreads / 32];
     const int p = first + blockIdx.x;
     const float *A = amplitudes + (size_t)p * n;
@@ -72,23 +70,7 @@ __global__ void __launch_bounds__(kProjectThreads) mixed_project_kernel(double2 
             intensity += f.x * f.x + f.y * f.y;
         }
         const double measured = (double)A[k];
-        double factor;
-        if (modulus_in_range<double>(intensity, measured)) {
-            double amplitude, ratio;
-            modulus_and_ratio(intensity, measured, amplitude, ratio);
-            err += (measured - amplitude) * (measured - amplitude);
-            factor = (ratio - 1.0) * inv_n;
-        } else if (const double amplitude = sqrt(intensity); amplitude == 0.0) {
-            err += zero_infinite ? (double)INFINITY : measured * measured;
-            factor = 0.0;
-        } else {
-            err += (measured - amplitude) * (measured - amplitude);
-            factor = (measured / amplitude - 1.0) * inv_n;
-        }
-        if (factors) {
-            factors[(size_t)p * n + k] = factor;
-            continue;
-        }
+        const double factor = mixed_factor(intensity, measured, inv_n, zero_infinite != 0, err);
         for (int s = 0; s < states; s++) {
             double2 *f = dpsi + ((size_t)s * count + p) * n + k;
             f->x *= factor;
@@ -235,7 +217,7 @@ cudaError_t launch_mixed_position_pass(const MixedPassArgs &a, const Fft2Plan64 
             e = launch_fft2_f64(fft, a.dpsi + ((size_t)st * a.count + first) * n, m, false, s);
         if (e == cudaSuccess) {
             mixed_project_kernel<<<m, kProjectThreads, 0, s>>>(a.dpsi, a.amplitudes, first, a.count, a.states, n,
-                                                               1.0 / n, a.zero_pixel_infinite, a.error, nullptr);
+                                                               1.0 / n, a.zero_pixel_infinite, a.error);
             e = cudaGetLastError();
             count++;
         }
@@ -245,14 +227,6 @@ cudaError_t launch_mixed_position_pass(const MixedPassArgs &a, const Fft2Plan64 
     }
     if (launches) *launches = count;
     return cudaSuccess;
-}
-
-cudaError_t launch_mixed_factors(const double2 *dpsi, const float *amplitudes, int count, int states, int n,
-                                 bool zero_pixel_infinite, double *error, double *factors, cudaStream_t s) {
-    if (count <= 0) return cudaSuccess;
-    mixed_project_kernel<<<count, kProjectThreads, 0, s>>>(const_cast<double2 *>(dpsi), amplitudes, 0, count, states, n,
-                                                           1.0 / n, zero_pixel_infinite ? 1 : 0, error, factors);
-    return cudaGetLastError();
 }
 
 cudaError_t launch_orthogonalize(double2 *probes, int states, int n, double2 *gram, double2 *mixing, double2 *scratch,

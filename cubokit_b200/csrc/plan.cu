@@ -321,8 +321,6 @@ struct cubo_ptycho_plan {
     // (persistent, every item at once) launches instead of its own
     bool grouped_pass = false, grouped_gathers = false;
     std::vector<int> band_tile_offsets;  // [bands + 1]: band b's object-gather tiles are band_tiles[offsets[b] ..]
-    bool plane128 = false;  // FP64 128 x 128 planes: FFT, pointwise step and inverse FFT in one clustered launch
-    int plane_cluster = 2;  // CTAs per plane of that launch
     int states = 1;         // probe states (the mixed-state engine; 1 = single slice)
     int slices = 1;         // object slices (the multislice engine)
     bool multislice = false;        // the multislice engine (its iteration, even with one slice)
@@ -356,6 +354,8 @@ struct cubo_ptycho_plan {
     DeviceBuffer amplitudes, rr, cc, cls, tile_start, tile_list;
     DeviceBuffer object, grad_o, weight_o, tile_max;
     DeviceBuffer dpsi, error, errors, iteration;
+    bool rowcol64 = false, rowcol_positions = false;  // FP64 planes / position correction by rows and columns
+    DeviceBuffer position_terms64;
     bool fused_shift = false;  // the shift table in one launch (shift.cu)
     DeviceBuffer probe64, scratch64, spectrum64, shifted, shift_tmp64, ramps_r64, ramps_c64;
     DeviceBuffer partial_grad, partial_weight, grad_p64, weight_p64, probe_block_max;
@@ -366,7 +366,6 @@ struct cubo_ptycho_plan {
     DeviceBuffer gram64, mixing64, ortho64;
     DeviceBuffer waves64, props64, ident, slice_max;  // multislice: entering waves, propagators, identity classes
     DeviceBuffer prop_factors64;  // multislice, 128 x 128 planes: per gap the row and the column factor (128 + 128)
-    DeviceBuffer mixed_factors64;  // mixed state, 128 x 128 planes: the projection's factor per position and pixel
     DeviceBuffer tile_counts;          // position correction: candidate counts per tile, rebuilt on the device
     DeviceBuffer band_tiles, dpsi_band;  // banded iterations: tiles per band, the residuals of one band
     DeviceBuffer shard_loss, shard_counter;  // sharded iterations: this plan's summed squared error, its reduce counter
@@ -713,11 +712,8 @@ void build_plan(cubo_ptycho_plan *p, const cubo_ptycho_problem *pr) {
     p->error_count = p->fast     ? (long long)P * fast128_partials_per_position()
                      : p->bf16     ? (long long)P * bf16_partials_per_position()
                      : p->global32 ? (long long)P * global32_partials_per_position(p->R, p->C)
+                     : p->rowcol64 ? (long long)P * rowcol64_parts(p->R, p->C, p->states)
                                    : P;
-    if (p->plane128) {
-        check(p->fault.alloc(sizeof(int)), "cudaMalloc");
-        check(cudaMemsetAsync(p->fault.ptr, 0, sizeof(int), s), "memset");
-    }
     if (p->bf16) {
         // the real factor C of the 128-point DFT matrix (row 0 = 1, row 1 = cos(pi k), rows 2j, 2j + 1 = cos, sin of
         // 2 pi j k / 128) and C_sigma (its columns in the kernel's stage-4 order), split into bf16 hi + lo in FP64:
@@ -791,7 +787,7 @@ Fft2Plan64 fft64(const cubo_ptycho_plan *p) {
 
 // After a synchronize: a device wait that ran out (split-BF16 kernel) turns into CUBO_PTYCHO_DEVICE_TIMEOUT.
 void check_fault(cubo_ptycho_plan *p) {
-    if (!p->bf16 && !p->plane128) return;
+    if (!p->bf16) return;
     int f = 0;
     check(cudaMemcpy(&f, p->fault.ptr, sizeof(int), cudaMemcpyDeviceToHost), "read fault flag");
     if (f) {
@@ -815,33 +811,45 @@ void ensure_errors(cubo_ptycho_plan *p, long long needed) {
     p->errors_capacity = cap;
 }
 
-// A clustered 128 x 128 plane launch (FP64) over every position: the fields every use shares.
-Plane128Args plane_args(const cubo_ptycho_plan *p, int mode) {
-    Plane128Args a{};
-    a.mode = mode; a.first = 0; a.count = p->P; a.in_kind = kInputByPosition;
-    a.scan = ScanTables{p->rr.as<int>(), p->cc.as<int>(), p->cls.as<int>()};
-    a.object_rows = p->OR; a.object_columns = p->OC; a.pointwise = kPointwiseNone; a.scale = 1.0 / p->n;
-    a.amplitudes = p->amplitudes.as<float>(); a.error = p->error.as<double>(); a.inv_n = 1.0 / p->n;
-    a.tw = p->tw_r64.as<double2>(); a.out_stride = 1; a.out_offset = 0; a.fault = p->fault.as<int>();
-    a.ahead = p->sms / 2;  // the clusters resident at once (Q / 2 CTAs per SM, Q per cluster)
-    return a;
+// The geometry of the FP64 row and column launches (rowcol64.cu).
+RcGeometry rc_geometry(const cubo_ptycho_plan *p) {
+    return RcGeometry{p->R, p->C, p->OR, p->OC, ScanTables{p->rr.as<int>(), p->cc.as<int>(), p->cls.as<int>()},
+                      p->tw_r64.as<double2>(), p->tw_c64.as<double2>()};
 }
 
-void enqueue_plane(cubo_ptycho_plan *p, Kind kind, const Plane128Args &a) {
-    timed(p, kind, 1, [&] { return launch_plane128(a, p->plane_cluster, p->ctx->stream); });
+// Every position's planes through rows, columns and inverse rows: `in` (by class or by position) times the object patch
+// (conjugated) -> FFT -> the pointwise step of `step` (its planes are set here) -> inverse FFT -> out, `layers` planes a
+// position in_layer / out_layer apart.
+void enqueue_rowcol(cubo_ptycho_plan *p, Kind kind, const double2 *in, bool by_class, long long in_layer,
+                    const double2 *object, bool conj_object, RcColumns step, double2 *out, long long out_layer, int layers) {
+    RcRows r{};
+    r.in = in; r.by_class = by_class ? 1 : 0; r.in_layer = in_layer; r.object = object; r.conj_object = conj_object ? 1 : 0;
+    r.out = out; r.out_layer = out_layer; r.out_stride = p->n; r.count = p->P; r.layers = layers;
+    step.planes = out; step.layer = out_layer; step.stride = p->n; step.count = p->P; step.layers = layers;
+    timed(p, kind, 3, [&] {
+        const RcGeometry q = rc_geometry(p);
+        cudaError_t e = launch_rc_rows(q, r, false, p->ctx->stream);
+        if (e == cudaSuccess) e = launch_rc_columns(q, step, p->ctx->stream);
+        if (e == cudaSuccess) e = launch_rc_rows(q, r, true, p->ctx->stream);
+        return e;
+    });
 }
 
-// The full plane launch of every position: `in` (by class or by position) times the object patch (conjugated), FFT,
-// the propagator factors x 1/n (project == false) or the modulus projection with the error (project == true),
-// inverse FFT, into `out`.
-void enqueue_plane128(cubo_ptycho_plan *p, Kind kind, const double2 *in, bool by_class, const double2 *object,
-                      bool conj_object, bool project, const double2 *prop_factors, bool conj_prop, double2 *out) {
-    Plane128Args a = plane_args(p, kPlaneFull);
-    a.in = in; a.in_kind = by_class ? kInputByClass : kInputByPosition; a.object = object;
-    a.conj_object = conj_object ? 1 : 0; a.pointwise = project ? kPointwiseProjection : kPointwiseFactors;
-    a.prop_rows = prop_factors; a.prop_columns = prop_factors ? prop_factors + 128 : nullptr;
-    a.conj_prop = conj_prop ? 1 : 0; a.out = out;
-    enqueue_plane(p, kind, a);
+// The projection step of the position pass.
+RcColumns rc_projection(const cubo_ptycho_plan *p) {
+    RcColumns c{};
+    c.amplitudes = p->amplitudes.as<float>();
+    c.error = p->error.as<double>();
+    c.zero_infinite = p->zero_pixel_infinite ? 1 : 0;
+    return c;
+}
+// Multislice: the propagator of gap `gap`.
+RcColumns rc_propagation(const cubo_ptycho_plan *p, int gap, bool conjugate) {
+    RcColumns c{};
+    c.prop_rows = p->prop_factors64.as<double2>() + (size_t)gap * (p->R + p->C);
+    c.prop_columns = c.prop_rows + p->R;
+    c.conj_prop = conjugate ? 1 : 0;
+    return c;
 }
 
 // The shift table of probe state `st`.
@@ -1008,26 +1016,11 @@ void enqueue_position_pass(cubo_ptycho_plan *p) {
         fa.tw128 = p->tw_r.as<float2>();
         fa.partial_grad = p->partial_grad.as<float2>(); fa.partial_weight = p->partial_weight.as<float>();
         timed(p, kPositionPass, 1, [&] { return launch_fast128(fa, p->sms, s); });
-    } else if (p->states > 1 && p->plane128) {
-        if constexpr (std::is_same<T, double>::value) {  // every state's far field, the summed projection, inverses
-            for (int st = 0; st < p->states; st++) {
-                Plane128Args a = plane_args(p, kPlaneForward);
-                a.in = p->shifted.as<double2>() + (size_t)st * p->classes * n; a.in_kind = kInputByClass;
-                a.object = p->object.as<double2>(); a.out = p->dpsi.as<double2>() + (size_t)st * p->P * n;
-                enqueue_plane(p, kPositionPass, a);
-            }
-            timed(p, kPositionPass, 1, [&] {
-                return launch_mixed_factors(p->dpsi.as<double2>(), p->amplitudes.as<float>(), p->P, p->states, n,
-                                            p->zero_pixel_infinite, p->error.as<double>(),
-                                            p->mixed_factors64.as<double>(), s);
-            });
-            for (int st = 0; st < p->states; st++) {  // each state's residual: its far field x the common factor
-                Plane128Args a = plane_args(p, kPlaneInverse);
-                a.in = p->dpsi.as<double2>() + (size_t)st * p->P * n; a.out = const_cast<double2 *>(a.in);
-                a.pointwise = kPointwiseFactorPlane; a.factors = p->mixed_factors64.as<double>();
-                enqueue_plane(p, kPositionPass, a);
-            }
-        }
+    } else if (p->rowcol64) {
+        if constexpr (std::is_same<T, double>::value)
+            enqueue_rowcol(p, kPositionPass, p->shifted.as<double2>(), true, (long long)p->classes * n,
+                           p->object.as<double2>(), false, rc_projection(p), p->dpsi.as<double2>(),
+                           (long long)p->P * n, p->states);
     } else if (p->states > 1) {
         if constexpr (std::is_same<T, double>::value) {
             MixedPassArgs ma{};
@@ -1041,10 +1034,6 @@ void enqueue_position_pass(cubo_ptycho_plan *p) {
             p->launches += count;
             if (p->timing) p->kind_launches[kPositionPass] += count;
         }
-    } else if (p->plane128) {
-        if constexpr (std::is_same<T, double>::value)
-            enqueue_plane128(p, kPositionPass, p->shifted.as<double2>(), true, p->object.as<double2>(), false, true,
-                             nullptr, false, p->dpsi.as<double2>());
     } else if (p->global64) {
         int count = 0;
         if constexpr (std::is_same<T, double>::value) {
@@ -1195,24 +1184,26 @@ void enqueue_position_correction(cubo_ptycho_plan *p) {
     const ScanTables scan{p->rr.as<int>(), p->cc.as<int>(), p->cls.as<int>()};
     for (int first = 0; first < p->P; first += p->correction_chunk) {
         const int m = std::min(p->correction_chunk, p->P - first);
-        if (p->plane128) {
-            // the forward model's far field and the updated object's one row further (two forward plane launches),
-            // then the one column further with the solve of every position in the same launch
-            for (int v = 0; v < 3; v++) {
-                Plane128Args a = plane_args(p, kPlaneForward);
-                a.first = first; a.count = m; a.in = p->shifted.as<double2>(); a.in_kind = kInputByClass;
-                a.object = v == 0 ? p->object_before.as<double2>() : p->object.as<double2>();
-                a.object_row_offset = v == 1 ? 1 : 0; a.object_column_offset = v == 2 ? 1 : 0;
-                a.out = p->far64.as<double2>(); a.out_stride = 2; a.out_offset = v - 2LL * first;
-                if (v == 2) {
-                    a.pointwise = kPointwiseSolve; a.out_offset = 0; a.far = p->far64.as<double2>();
-                    a.positions = p->positions64.as<double>(); a.initial = p->initial64.as<double>();
-                    a.position_count = p->P; a.position_step_size = p->params.position_step_size;
-                    a.limit_update = p->limit_update; a.limit_total = p->limit_total;
-                    a.position_bad = p->position_bad.as<int>();
-                }
-                enqueue_plane(p, kPositionCorrection, a);
-            }
+        if (p->rowcol_positions) {
+            // the far fields of the object before the update at the centre and after it a row and a column further, whose
+            // columns go straight into the normal equations
+            RcRows r{};
+            r.in = p->shifted.as<double2>(); r.by_class = 1; r.object = p->object_before.as<double2>();
+            r.object_after = p->object.as<double2>(); r.out = p->far64.as<double2>(); r.out_layer = p->n;
+            r.out_stride = 3LL * p->n; r.out_first = first; r.first = first; r.count = m; r.layers = 3;
+            RcColumns c{};
+            c.planes = r.out; c.layer = r.out_layer; c.stride = r.out_stride; c.plane_first = first; c.first = first;
+            c.count = m; c.layers = 3; c.amplitudes = p->amplitudes.as<float>(); c.terms = p->position_terms64.as<double>();
+            timed(p, kPositionCorrection, 3, [&] {
+                const RcGeometry q = rc_geometry(p);
+                cudaError_t e = launch_rc_rows(q, r, false, s);
+                if (e == cudaSuccess) e = launch_rc_columns(q, c, s);
+                if (e == cudaSuccess)
+                    e = launch_rc_move(c.terms, rowcol64_parts(p->R, p->C, 3), first, m, p->positions64.as<double>(),
+                                       p->initial64.as<double>(), p->P, p->params.position_step_size, p->limit_update,
+                                       p->limit_total, p->position_bad.as<int>(), s);
+                return e;
+            });
             continue;
         }
         timed(p, kPositionCorrection, 3, [&] {
@@ -1293,15 +1284,15 @@ void enqueue_multislice_iteration(cubo_ptycho_plan *p) {
     const ScanTables own{p->rr.as<int>(), p->cc.as<int>(), p->ident.as<int>()};  // class p = position p
     double2 *obj = p->object.as<double2>(), *chi = p->dpsi.as<double2>(), *waves = p->waves64.as<double2>();
     const double2 *shifted = p->shifted.as<double2>(), *props = p->props64.as<double2>();
-    const double2 *factors = p->prop_factors64.as<double2>();
     const Fft2Plan64 f = fft64(p);
     enqueue_shift_table<double>(p);
-    if (p->plane128) {  // forward and detector, one plane launch per slice
+    if (p->rowcol64) {
         for (int sl = 0; sl < L; sl++) {
             const double2 *in = sl == 0 ? shifted : waves + (size_t)(sl - 1) * planes;
             const bool last = sl == L - 1;
-            enqueue_plane128(p, kPositionPass, in, sl == 0, obj + (size_t)sl * plane, false, last,
-                             last ? nullptr : factors + (size_t)sl * 256, false, last ? chi : waves + (size_t)sl * planes);
+            enqueue_rowcol(p, kPositionPass, in, sl == 0, 0, obj + (size_t)sl * plane, false,
+                           last ? rc_projection(p) : rc_propagation(p, sl, false),
+                           last ? chi : waves + (size_t)sl * planes, 0, 1);
         }
     } else {
     // forward (:503-515): exit_s = wave_s x O_s; wave_{s+1} = IFFT(FFT(exit_s) x prop_s / n)
@@ -1350,9 +1341,9 @@ void enqueue_multislice_iteration(cubo_ptycho_plan *p) {
         ga.tile_max = p->tile_max.as<double>() + (size_t)sl * p->gather_maxima;
         timed(p, kObjectGather, p->gather_groups > 1 ? 2 : 1, [&] { return gather_object<double>(p, ga); });
         if (sl == 0) break;
-        if (p->plane128) {
-            enqueue_plane128(p, kBackPropagation, chi, false, obj + (size_t)sl * plane, true, false,
-                             factors + (size_t)(sl - 1) * 256, true, chi);
+        if (p->rowcol64) {
+            enqueue_rowcol(p, kBackPropagation, chi, false, 0, obj + (size_t)sl * plane, true,
+                           rc_propagation(p, sl - 1, true), chi, 0, 1);
             continue;
         }
         timed(p, kBackPropagation, 6, [&] {
@@ -1695,12 +1686,11 @@ int create_plan(cubo_ptycho_context *ctx, const cubo_ptycho_problem *pr, const c
         // FP64 planes too large for one CTA go through global memory (any size the line transform takes)
         p->global64 = p->fp64 && (!smem_pass || pp->variant == CUBO_PTYCHO_VARIANT_GLOBAL || p->states > 1 ||
                                   p->multislice);
-        // 128 x 128 FP64 planes: the clustered plane launches (not with the generic variant)
-        p->plane128 = p->global64 && p->R == 128 && p->C == 128 && pp->variant != CUBO_PTYCHO_VARIANT_GENERIC;
-        if (p->plane128) {
-            check(configure_plane128(), "configure plane transform");
-            p->plane_cluster = plane128_cluster();
-        }
+        // FP64 planes through row and column launches (not with the generic variant, which keeps the batched line transforms)
+        const bool rc = p->fp64 && pp->variant != CUBO_PTYCHO_VARIANT_GENERIC;
+        p->rowcol64 = rc && p->global64 && rowcol64_applicable(p->R, p->C, p->states);
+        p->rowcol_positions = rc && pp->has_position_correction && rowcol64_applicable(p->R, p->C, 3);
+        if (p->rowcol64 || p->rowcol_positions) check(configure_rowcol64(), "configure row and column launches");
         // FP32 planes too large for one CTA (or any size with the global variant): rows and columns through global memory
         p->global32 = !p->fp64 && pp->form != CUBO_PTYCHO_FORM_SPLIT_BF16 &&
                       (!smem_pass || pp->variant == CUBO_PTYCHO_VARIANT_GLOBAL) && global32_applicable(p->R, p->C);
@@ -1740,11 +1730,9 @@ int create_plan(cubo_ptycho_context *ctx, const cubo_ptycho_problem *pr, const c
         p->correct_positions = pp->has_position_correction != 0;  // before the scan tables: one class per position
         if (p->fp64) build_plan<double>(p, pr);
         else build_plan<float>(p, pr);
-        if (p->plane128 && p->states > 1)
-            check(p->mixed_factors64.alloc((size_t)p->P * p->n * sizeof(double)), "cudaMalloc mixed-state factors");
         if (p->multislice && p->slices > 1) {
             upload(p->props64, props, ctx->stream);
-            if (p->plane128)
+            if (p->rowcol64)
                 upload(p->prop_factors64,
                        fresnel_factors(p->R, p->C, multi->row_sampling, multi->column_sampling, multi->wavelength,
                                        p->slices - 1, multi->slice_thicknesses),
@@ -1768,12 +1756,13 @@ int create_plan(cubo_ptycho_context *ctx, const cubo_ptycho_problem *pr, const c
             check(p->object_before.alloc((size_t)p->objects * sizeof(double2)), "cudaMalloc");
             check(p->position_bad.alloc(sizeof(int)), "cudaMalloc");
             check(cudaMemsetAsync(p->position_bad.ptr, 0, sizeof(int), ctx->stream), "memset");
-            // far fields per position, FP64 (three; two with the clustered plane launches, which solve with the
-            // third on chip): chunks of at most 1 GiB (2 GiB)
-            const size_t per_position = (size_t)(p->plane128 ? 2 : 3) * p->n * sizeof(double2);
-            const size_t budget = p->plane128 ? (2ull << 30) : (1ull << 30);
+            // three far fields per position, FP64: chunks of at most 1 GiB
+            const size_t per_position = 3 * (size_t)p->n * sizeof(double2), budget = 1ull << 30;
             p->correction_chunk = (int)std::max<size_t>(1, std::min<size_t>(p->P, budget / per_position));
             check(p->far64.alloc((size_t)p->correction_chunk * per_position), "cudaMalloc");
+            if (p->rowcol_positions)
+                check(p->position_terms64.alloc((size_t)p->correction_chunk * rowcol64_parts(p->R, p->C, 3) * 5 *
+                                                sizeof(double)), "cudaMalloc");
         }
         check(cudaStreamSynchronize(ctx->stream), "plan upload");
     });
@@ -2336,7 +2325,7 @@ void build_groups(cubo_ptycho_batch *b) {
         if (p->states != 1 || p->multislice || p->banded || p->correct_positions) continue;
         if (p->fp64) ensure_dpsi<double>(p);
         else ensure_dpsi<float>(p);
-        const bool generic_pass = p->fp64 ? !p->global64 && !p->plane128 : !p->fast && !p->bf16 && !p->global32;
+        const bool generic_pass = p->fp64 ? !p->global64 : !p->fast && !p->bf16 && !p->global32;
         if (generic_pass && position_pass_groupable(p->R, p->C, p->fp64)) {
             add(0, p, p->R, p->params.pass_shape, p->P);
             p->grouped_pass = true;

@@ -6,18 +6,21 @@
 
 namespace cubo {
 
-// Adds one detector pixel's terms to v = [sum dx dx, sum dx dy, sum dy dy, sum dx difference, sum dy difference]:
-// f the forward model's far field, gx / gy the far fields of the updated object one row / one column further,
-// measured the amplitude.
-__device__ __forceinline__ void position_terms(double2 f, double2 gx, double2 gy, double measured, double (&v)[5]) {
-    const double difference = measured * measured - (f.x * f.x + f.y * f.y);
-    const double dx = 2 * ((f.x - gx.x) * f.x + (f.y - gx.y) * f.y);
-    const double dy = 2 * ((f.x - gy.x) * f.x + (f.y - gy.y) * f.y);
+// The products of one detector pixel's derivatives and intensity difference, added to v (position_terms).
+__device__ __forceinline__ void position_products(double dx, double dy, double difference, double (&v)[5]) {
     v[0] += dx * dx;
     v[1] += dx * dy;
     v[2] += dy * dy;
     v[3] += dx * difference;
     v[4] += dy * difference;
+}
+
+// Adds one detector pixel's terms to v = [sum dx dx, sum dx dy, sum dy dy, sum dx difference, sum dy difference]:
+// f the forward model's far field, gx / gy the far fields of the updated object one row / one column further,
+// measured the amplitude.
+__device__ __forceinline__ void position_terms(double2 f, double2 gx, double2 gy, double measured, double (&v)[5]) {
+    position_products(2 * ((f.x - gx.x) * f.x + (f.y - gx.y) * f.y), 2 * ((f.x - gy.x) * f.x + (f.y - gy.y) * f.y),
+                      measured * measured - (f.x * f.x + f.y * f.y), v);
 }
 
 // Cramer's rule on the summed terms, the step, the per-update and total limits (in pixels; infinite = none), then the

@@ -83,4 +83,23 @@ __device__ __forceinline__ void project_values(C2<T> (&x)[R], const float (&meas
     }
 }
 
+// The mixed states' common factor of a pixel of summed intensity `power`, (A / sqrt(power) - 1) / n, and its squared error;
+// a zero intensity has factor 0 and adds an infinite term or, on request, A^2 (PtychographyEngines.swift:188-195).
+__device__ __forceinline__ double mixed_factor(double power, double measured, double inv_n, bool zero_infinite,
+                                               double &err) {
+    double modulus, ratio;
+    if (modulus_in_range<double>(power, measured)) {
+        modulus_and_ratio(power, measured, modulus, ratio);
+    } else {
+        modulus = sqrt(power);
+        if (modulus == 0.0) {
+            err += zero_infinite ? __longlong_as_double(0x7ff0000000000000ll) : measured * measured;
+            return 0.0;
+        }
+        ratio = measured / modulus;
+    }
+    err += (measured - modulus) * (measured - modulus);
+    return (ratio - 1.0) * inv_n;
+}
+
 }  // namespace cubo
