@@ -109,7 +109,7 @@ struct Bf16Args {
     float2 *dpsi;              // [positions - dpsi_first][row][column]
     int dpsi_first;            // the position whose residual dpsi[0] holds (a band's first, or 0)
     double *error;             // [positions][bf16_partials_per_position()]
-    const uint16_t *c_planes;  // [4][128][128] bf16 bits: C hi, C lo, C_sigma hi, C_sigma lo (rows m, columns k)
+    const uint16_t *c_planes;  // [2][128][128] bf16 bits: C_sigma hi, C_sigma lo (rows m, columns k)
     int *fault;                // set when a device wait ran out
 };
 bool bf16_applicable(int rows, int columns);

@@ -716,24 +716,21 @@ void build_plan(cubo_ptycho_plan *p, const cubo_ptycho_problem *pr) {
                                    : P;
     if (p->bf16) {
         // the real factor C of the 128-point DFT matrix (row 0 = 1, row 1 = cos(pi k), rows 2j, 2j + 1 = cos, sin of
-        // 2 pi j k / 128) and C_sigma (its columns in the kernel's stage-4 order), split into bf16 hi + lo in FP64:
-        // planes C hi, C lo, C_sigma hi, C_sigma lo, [m][k]
+        // 2 pi j k / 128), its columns in the kernel's contraction order, split into bf16 hi + lo in FP64: planes hi, lo,
+        // [m][k]
         auto c_value = [&](int m, int k) -> double {
             if (m == 0) return 1.0;
             if (m == 1) return (k & 1) ? -1.0 : 1.0;
             const double a = 2.0 * kPi * (double)(((m >> 1) * k) % R) / (double)R;
             return (m & 1) ? std::sin(a) : std::cos(a);
         };
-        std::vector<uint16_t> planes(4 * (size_t)n);
+        std::vector<uint16_t> planes(2 * (size_t)n);
         for (int m = 0; m < R; m++)
             for (int k = 0; k < C; k++) {
-                const double v[2] = {c_value(m, k), c_value(m, bf16_sigma(k))};
-                for (int part = 0; part < 2; part++) {
-                    const uint16_t hi = bf16_round(v[part]);
-                    const uint16_t lo = bf16_round(v[part] - bf16_to_double(hi));
-                    planes[(size_t)(2 * part) * n + m * C + k] = hi;
-                    planes[(size_t)(2 * part + 1) * n + m * C + k] = lo;
-                }
+                const double v = c_value(m, bf16_sigma(k));
+                const uint16_t hi = bf16_round(v);
+                planes[m * C + k] = hi;
+                planes[(size_t)n + m * C + k] = bf16_round(v - bf16_to_double(hi));
             }
         upload(p->c_planes, planes, s);
         check(p->fault.alloc(sizeof(int)), "cudaMalloc");

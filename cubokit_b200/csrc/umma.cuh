@@ -69,6 +69,11 @@ __device__ __forceinline__ void mbar_init(uint64_t *mbar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(mbar)), "r"(count) : "memory");
 }
 
+// One arrival on *mbar (release at CTA scope).
+__device__ __forceinline__ void mbar_arrive(uint64_t *mbar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(mbar)) : "memory");
+}
+
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *mbar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
