@@ -12,12 +12,14 @@
 //                 z = sqrt(3) - 2 (Unser, Aldroubi & Eden, IEEE Trans. Signal Process. 41(2), 1993) with periodic
 //                 states, O(n) per line in FP64, no transform needed.
 //
-// One CTA of 1024 threads per pattern at a time (grid-stride over patterns, one CTA per SM).  While a pattern is
+// Cubic patterns whose sides are multiples of 16 keep both axes in registers (prepare_spline_kernel).  The rest: one CTA of
+// 1024 threads per pattern at a time (grid-stride over patterns, one CTA per SM).  While a pattern is
 // computed, the next one is copied into shared memory with cp.async.  The arithmetic is FP64 up to the square root of
 // the Float32 output.  Every output pixel has the pattern's own fractional offsets, so the 2-D weights are a product
 // of per-axis weights and the interpolation is separable: each thread walks down one column with the last few
 // row-interpolated values in registers.  Each warp writes its sums of a pattern (fixed order), and a fixed-order sum
 // runs over them afterwards: the same inputs give the same bits, however the patterns are split into launches.
+#include <algorithm>
 #include <cfloat>
 
 #include "engine.h"
@@ -399,6 +401,184 @@ __global__ void __launch_bounds__(kPrepThreads) prepare_kernel(const float *cube
     }
 }
 
+// ---- cubic, sides of whole segments: both axes in registers
+
+constexpr int kSplineThreads = 512;  // most threads a CTA: 128 registers each, no spills
+
+// The states entering a warp's segments.  Lanes `stride` apart hold the segments g = 0 .. segs - 1 of one line (segment 0 at
+// lane `base`); `end` is the segment's end value from a zero state.  Returns the true entering state: what the segments before
+// (kReverse: after) carry in, and the periodic state: the line's own end times carry, gain^(segments before) / (1 - z^n).
+template <bool kReverse>
+__device__ __forceinline__ double entering_state(double end, int g, int segs, int lane, int stride, double gain, double carry) {
+    const int order = kReverse ? segs - 1 - g : g;  // segments before this one
+    double s = end, power = gain;
+    for (int d = 1; d < segs; d *= 2) {  // inclusive scan of s[order] = end[order] + gain s[order - 1]
+        const double other = __shfl_sync(0xffffffffu, s, lane + (kReverse ? d : -d) * stride);
+        if (order >= d) s = fma(power, other, s);
+        power *= power;
+    }
+    const int line = lane - g * stride;
+    const double whole = __shfl_sync(0xffffffffu, s, line + (kReverse ? 0 : segs - 1) * stride);
+    const double before = __shfl_sync(0xffffffffu, s, lane + (kReverse ? 1 : -1) * stride);
+    return fma(carry, whole, order > 0 ? before : 0.0);
+}
+
+// One segment's kSegMax samples -> its values h[k] = sum_b w[b] c[k + b] of the line's spline coefficients c (over 6), the
+// three coefficients past the segment taken from the next one's lane.
+__device__ __forceinline__ void spline_segment(double (&v)[kSegMax], const double (&w)[4], int g, int segs, int lane,
+                                               int stride, double gain, double carry, double carry_back) {
+    constexpr double z = kPole;
+    double y = 0.0;
+#pragma unroll
+    for (int k = 0; k < kSegMax; k++) {
+        y = v[k] + z * y;
+        v[k] = y;
+    }
+    const double e = entering_state<false>(y, g, segs, lane, stride, gain, carry);
+    double u = 0.0;
+#pragma unroll
+    for (int k = kSegMax - 1; k >= 0; k--) {
+        u = z * (u - (v[k] + kZ.v[k + 1] * e));
+        v[k] = u;
+    }
+    const double f = entering_state<true>(u, g, segs, lane, stride, gain, carry_back);
+#pragma unroll
+    for (int k = 0; k < kSegMax; k++) v[k] += kZ.v[kSegMax - k] * f;
+    double halo[3];
+    const int next = lane + (g == segs - 1 ? -g : 1) * stride;
+#pragma unroll
+    for (int k = 0; k < 3; k++) halo[k] = __shfl_sync(0xffffffffu, v[k], next);
+#pragma unroll
+    for (int k = 0; k < kSegMax; k++) {
+        double h = 0.0;
+#pragma unroll
+        for (int b = 0; b < 4; b++) h += w[b] * (k + b < kSegMax ? v[(k + b) % kSegMax] : halo[(k + b) % kSegMax % 3]);
+        v[k] = h;
+    }
+}
+
+// The plane between the axes, in doubles: 16 columns and 2 of padding, rows an odd number apart, and 4 more after each 16
+// rows, so that neither the rows' stores (a few rows, every 16th column) nor the columns' loads (four columns, every 16th
+// row) meet in a bank.
+__host__ __device__ __forceinline__ int spline_pitch(int columns) { return columns + 2 * (columns / kSegMax) + 1; }
+__host__ __device__ __forceinline__ int spline_plane(int rows, int columns) {
+    return (rows * spline_pitch(columns) + 4 * (rows / kSegMax) + 1) & ~1;
+}
+
+// Cubic shift of patterns whose sides are multiples of kSegMax: prefilter and interpolation of an axis follow one another in
+// the registers of the threads that hold its segments (the shift is one number for a pattern, so the taps of a segment are
+// its own coefficients and three of the next), rows first, then columns, whose results leave as they are.  A warp holds whole
+// lines, so segments exchange by shuffles: two block barriers a pattern in place of seven, one store and one load of shared
+// memory a value in place of two and seven.  Bound by FP64 and issue: 16,384 patterns of 128 x 128 1.375 -> 1.29 ms,
+// 12,000 of 112 x 128 1.41 -> 1.03, of 96 x 96 1.08 -> 0.91 and of 64 x 64, several CTAs an SM, 0.75 -> 0.30 (every size below
+// the limit was quicker this way; 1024 threads of 64 registers spilled: 1.55 ms at 128 x 128).
+// While the columns are computed, the next pattern is copied in, its 16-byte units swizzled for the rows' loads.
+template <int kRows, int kColumns>
+__global__ void __launch_bounds__(kSplineThreads) prepare_spline_kernel(const float *cube, int count, int rows_arg,
+                                                                      int columns_arg, const PatternShift *shifts,
+                                                                      float *amplitudes, double *sums, int *bad,
+                                                                      int aligned) {
+    extern __shared__ __align__(16) double smem[];
+    const int rows = kRows ? kRows : rows_arg, columns = kColumns ? kColumns : columns_arg;
+    const int n = rows * columns, pitch = spline_pitch(columns);
+    double *const plane = smem;
+    float *const staged = reinterpret_cast<float *>(smem + spline_plane(rows, columns));
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int row_segs = columns / kSegMax, column_segs = rows / kSegMax;  // segments of a row, of a column
+    const int row_lines = 32 / row_segs, column_lines = 32 / column_segs;  // lines a warp holds
+    // rows: segments in adjacent lanes; columns: lines in adjacent lanes
+    const int rg = lane % row_segs, rq = lane / row_segs, cq = lane % column_lines, cg = lane / column_lines;
+    const double gain = int_power(kPole, kSegMax);
+    const int cl = cg < column_segs ? cg : 0;
+    const double row_wrap = 1.0 / (1.0 - int_power(kPole, columns)), column_wrap = 1.0 / (1.0 - int_power(kPole, rows));
+    const double row_carry = row_wrap * int_power(gain, rg), row_back = row_wrap * int_power(gain, row_segs - 1 - rg);
+    const double column_carry = column_wrap * int_power(gain, cl);
+    const double column_back = column_wrap * int_power(gain, column_segs - 1 - cl);
+    auto copy = [&](int p) {
+        const float *src = cube + (size_t)p * n;
+        const uint32_t d = umma::smem_u32(staged);
+        if (aligned) {
+            for (int i = threadIdx.x; i < n / 4; i += blockDim.x) {
+                // eight lanes' loads of one unit of their segments: eight banks
+                const int at = i ^ (((i % (columns / 4)) >> 3) & 3);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16u * (uint32_t)at), "l"(src + 4 * (size_t)i)
+                             : "memory");
+            }
+        } else {
+            for (int i = threadIdx.x; i < n; i += blockDim.x) {
+                const int at = i ^ ((((i % columns) >> 5) & 3) << 2);
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d + 4u * (uint32_t)at), "l"(src + i) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if ((int)blockIdx.x < count) copy(blockIdx.x);
+    for (int p = blockIdx.x; p < count; p += gridDim.x) {
+        copy_pattern_wait();
+        const PatternShift sh = shifts[p];
+        double w[4], v[kSegMax];
+        cubic_weights(sh.column_fraction, w);
+        for (int first = warp * row_lines; first < rows; first += warps * row_lines) {
+            const int r = first + rq;
+            const bool active = rq < row_lines && r < rows;
+            const float4 *line = reinterpret_cast<const float4 *>(staged + (active ? r : 0) * columns) + 4 * rg;
+#pragma unroll
+            for (int k = 0; k < kSegMax / 4; k++) {
+                const float4 x = line[k ^ ((rg >> 1) & 3)];
+                v[4 * k] = x.x; v[4 * k + 1] = x.y; v[4 * k + 2] = x.z; v[4 * k + 3] = x.w;
+            }
+            spline_segment(v, w, rg, row_segs, lane, 1, gain, row_carry, row_back);
+            if (active) {  // h[k] is the value at column 16 g + k - dc: two runs, split where a multiple of 16 is passed
+                const int at = wrap_index(rg * kSegMax - (sh.column - 1), columns), low = at % kSegMax, block = at / kSegMax;
+                double *d = plane + r * pitch + 4 * (r / kSegMax) + low;
+                const int d0 = 18 * block, d1 = 18 * (block + 1 == row_segs ? 0 : block + 1) - kSegMax;
+#pragma unroll
+                for (int k = 0; k < kSegMax; k++) d[(k < kSegMax - low ? d0 : d1) + k] = v[k];
+            }
+        }
+        __syncthreads();
+        if (p + (int)gridDim.x < count) copy(p + gridDim.x);
+        cubic_weights(sh.row_fraction, w);
+#pragma unroll
+        for (int a = 0; a < 4; a++) w[a] *= 36.0;  // the factor 6 of both axes' coefficients
+        double total = 0.0, clipped = 0.0;
+        float *out = amplitudes + (size_t)p * n;
+        for (int first = warp * column_lines; first < columns; first += warps * column_lines) {
+            const int c = first + cq;
+            const bool active = cg < column_segs && c < columns;
+            const int cs = active ? c : 0;
+            const double *line = plane + cl * (kSegMax * pitch + 4) + cs + 2 * (cs / kSegMax);
+#pragma unroll
+            for (int k = 0; k < kSegMax; k++) v[k] = line[k * pitch];
+            spline_segment(v, w, cl, column_segs, lane, column_lines, gain, column_carry, column_back);
+            if (active) {
+                const int at = wrap_index(cl * kSegMax - (sh.row - 1), rows), low = rows - at;  // wraps before value `low`
+                const int d0 = at * columns + c, d1 = d0 - n;
+#pragma unroll
+                for (int k = 0; k < kSegMax; k++) {
+                    total += v[k];
+                    const double pos = v[k] > 0.0 ? v[k] : 0.0;
+                    clipped += pos;
+                    out[(k < low ? d0 : d1) + k * columns] = sqrtf((float)pos);
+                }
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            total += __shfl_down_sync(0xffffffffu, total, o);
+            clipped += __shfl_down_sync(0xffffffffu, clipped, o);
+        }
+        if (lane == 0) {
+            if (!(fabs(total) <= DBL_MAX)) atomicOr(bad, 1);  // a NaN or an infinity reaches every sum of its line
+            for (int i = warp; i < kPrepWarps; i += warps) {  // a smaller CTA's missing warps add nothing
+                double *d = sums + ((size_t)p * kPrepWarps + i) * 2;
+                d[0] = i == warp ? total : 0.0;
+                d[1] = i == warp ? clipped : 0.0;
+            }
+        }
+    }
+}
+
 // Fixed-order sums over the patterns: block b sums its slice of patterns (each pattern's warp sums in warp order), then
 // one block sums the blocks.
 __global__ void __launch_bounds__(1024) prepare_partial_kernel(const double *sums, int count, double *block_sums) {
@@ -459,6 +639,23 @@ bool prepare_can_stage(const float *cube, int rows, int columns, bool cubic, siz
 }
 }  // namespace
 
+namespace {
+// The register form's threads a CTA (as many warps as its longer pass can use) and shared memory, and whether it takes the
+// pattern: whole segments, a line within a warp, the plane and the next pattern in shared memory.
+int spline_threads(int rows, int columns) {
+    const int row_lines = 32 / (columns / kSegMax), column_lines = 32 / (rows / kSegMax);
+    const int a = (rows + row_lines - 1) / row_lines, b = (columns + column_lines - 1) / column_lines;
+    return 32 * std::min(kSplineThreads / 32, std::max(a, b));
+}
+size_t spline_smem(int rows, int columns) {
+    return (size_t)spline_plane(rows, columns) * sizeof(double) + (size_t)rows * columns * sizeof(float);
+}
+bool spline_applicable(int rows, int columns, size_t smem_limit) {
+    return rows % kSegMax == 0 && columns % kSegMax == 0 && rows <= 32 * kSegMax && columns <= 32 * kSegMax &&
+           spline_smem(rows, columns) <= smem_limit;
+}
+}  // namespace
+
 int prepare_max_line() { return kSegMax * kPrepThreads; }
 int prepare_scratch_doubles() { return 2 * kPrepSumBlocks + 2; }
 int prepare_sums_per_pattern() { return 2 * kPrepWarps; }
@@ -470,8 +667,11 @@ cudaError_t configure_prepare() {
     e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
     if (e != cudaSuccess) return e;
     const int limit = optin - 1024;
-    for (auto f : {prepare_kernel<false, 0, 0>, prepare_kernel<false, 128, 128>, prepare_kernel<true, 0, 0>,
-                   prepare_kernel<true, 128, 128>}) {
+    for (auto f : {prepare_kernel<false, 0, 0>, prepare_kernel<false, 128, 128>, prepare_kernel<true, 0, 0>}) {
+        e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+        if (e != cudaSuccess) return e;
+    }
+    for (auto f : {prepare_spline_kernel<0, 0>, prepare_spline_kernel<128, 128>}) {
         e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
         if (e != cudaSuccess) return e;
     }
@@ -481,15 +681,27 @@ cudaError_t configure_prepare() {
 cudaError_t launch_prepare(const float *cube, int count, int rows, int columns, const PatternShift *shifts, bool cubic,
                            float *amplitudes, double *sums, int *bad, int ctas, size_t smem_limit, cudaStream_t s) {
     if (count <= 0) return cudaSuccess;
+    const bool square128 = rows == 128 && columns == 128;
+    if (cubic && spline_applicable(rows, columns, smem_limit)) {
+        const int threads = spline_threads(rows, columns);
+        const size_t smem = spline_smem(rows, columns);
+        const size_t fit = std::min<size_t>(kSplineThreads / threads, smem_limit / (smem + 1024));
+        const int resident = (int)std::max<size_t>(1, fit);
+        auto kernel = square128 ? prepare_spline_kernel<128, 128> : prepare_spline_kernel<0, 0>;
+        const int aligned = ((uintptr_t)cube & 15) == 0;
+        kernel<<<std::min(count, ctas * resident), threads, smem, s>>>(cube, count, rows, columns, shifts, amplitudes, sums,
+                                                                       bad, aligned);
+        return cudaGetLastError();
+    }
     const int grid = count < ctas ? count : ctas;
     const bool staged = prepare_can_stage(cube, rows, columns, cubic, smem_limit);
     const int staged_at = staged ? (int)prepare_base_doubles(rows, columns, cubic) : -1;
     const int aligned_rows = columns % 4 == 0 && ((uintptr_t)amplitudes & 15) == 0;
     const size_t smem = prepare_smem(rows, columns, cubic, staged);
     // 128 x 128 patterns (the usual detector) have their own instantiation: constant strides and trip counts
-    const bool square128 = rows == 128 && columns == 128;
-    auto kernel = cubic ? (square128 ? prepare_kernel<true, 128, 128> : prepare_kernel<true, 0, 0>)
-                        : (square128 ? prepare_kernel<false, 128, 128> : prepare_kernel<false, 0, 0>);
+    auto kernel = cubic       ? prepare_kernel<true, 0, 0>
+                  : square128 ? prepare_kernel<false, 128, 128>
+                              : prepare_kernel<false, 0, 0>;
     kernel<<<grid, kPrepThreads, smem, s>>>(cube, count, rows, columns, shifts, amplitudes, sums, bad, staged_at,
                                             aligned_rows);
     return cudaGetLastError();
