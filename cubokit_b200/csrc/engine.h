@@ -301,6 +301,7 @@ struct RcRows {
     double2 *out;
     long long out_layer, out_stride;
     int out_first, first, count, layers;
+    const double2 *from;  // inverse: the spectrum, by position (null: out itself)
 };
 // Columns, in place in planes + layer `layer` + (p - plane_first) stride: with `terms` the normal equations of position
 // correction from three layers ([p - plane_first][rowcol64_parts][5], nothing written back), with prop_rows the separable
@@ -320,6 +321,8 @@ bool rowcol64_applicable(int rows, int columns, int layers);
 int rowcol64_parts(int rows, int columns, int layers);  // column CTAs of a position
 cudaError_t configure_rowcol64();
 cudaError_t launch_rc_rows(const RcGeometry &q, const RcRows &r, bool inverse, cudaStream_t s);
+// Inverse rows of r.in (by position) into r.out and, times the object patch, forward rows into next; r.in may be either.
+cudaError_t launch_rc_through(const RcGeometry &q, const RcRows &r, double2 *next, cudaStream_t s);
 cudaError_t launch_rc_columns(const RcGeometry &q, const RcColumns &c, cudaStream_t s);
 cudaError_t launch_rc_move(const double *terms, int per, int first, int m, double *positions, const double *initial,
                            int count, double step, double limit_update, double limit_total, int *bad, cudaStream_t s);

@@ -814,24 +814,6 @@ RcGeometry rc_geometry(const cubo_ptycho_plan *p) {
                       p->tw_r64.as<double2>(), p->tw_c64.as<double2>()};
 }
 
-// Every position's planes through rows, columns and inverse rows: `in` (by class or by position) times the object patch
-// (conjugated) -> FFT -> the pointwise step of `step` (its planes are set here) -> inverse FFT -> out, `layers` planes a
-// position in_layer / out_layer apart.
-void enqueue_rowcol(cubo_ptycho_plan *p, Kind kind, const double2 *in, bool by_class, long long in_layer,
-                    const double2 *object, bool conj_object, RcColumns step, double2 *out, long long out_layer, int layers) {
-    RcRows r{};
-    r.in = in; r.by_class = by_class ? 1 : 0; r.in_layer = in_layer; r.object = object; r.conj_object = conj_object ? 1 : 0;
-    r.out = out; r.out_layer = out_layer; r.out_stride = p->n; r.count = p->P; r.layers = layers;
-    step.planes = out; step.layer = out_layer; step.stride = p->n; step.count = p->P; step.layers = layers;
-    timed(p, kind, 3, [&] {
-        const RcGeometry q = rc_geometry(p);
-        cudaError_t e = launch_rc_rows(q, r, false, p->ctx->stream);
-        if (e == cudaSuccess) e = launch_rc_columns(q, step, p->ctx->stream);
-        if (e == cudaSuccess) e = launch_rc_rows(q, r, true, p->ctx->stream);
-        return e;
-    });
-}
-
 // The projection step of the position pass.
 RcColumns rc_projection(const cubo_ptycho_plan *p) {
     RcColumns c{};
@@ -1015,9 +997,19 @@ void enqueue_position_pass(cubo_ptycho_plan *p) {
         timed(p, kPositionPass, 1, [&] { return launch_fast128(fa, p->sms, s); });
     } else if (p->rowcol64) {
         if constexpr (std::is_same<T, double>::value)
-            enqueue_rowcol(p, kPositionPass, p->shifted.as<double2>(), true, (long long)p->classes * n,
-                           p->object.as<double2>(), false, rc_projection(p), p->dpsi.as<double2>(),
-                           (long long)p->P * n, p->states);
+            timed(p, kPositionPass, 3, [&] {  // every state's planes: rows, columns with the projection, inverse rows
+                const RcGeometry q = rc_geometry(p);
+                RcRows r{};
+                r.in = p->shifted.as<double2>(); r.by_class = 1; r.in_layer = (long long)p->classes * n;
+                r.object = p->object.as<double2>(); r.out = p->dpsi.as<double2>(); r.out_layer = (long long)p->P * n;
+                r.out_stride = n; r.count = p->P; r.layers = p->states;
+                RcColumns c = rc_projection(p);
+                c.planes = r.out; c.layer = r.out_layer; c.stride = n; c.count = p->P; c.layers = p->states;
+                cudaError_t e = launch_rc_rows(q, r, false, s);
+                if (e == cudaSuccess) e = launch_rc_columns(q, c, s);
+                if (e == cudaSuccess) e = launch_rc_rows(q, r, true, s);
+                return e;
+            });
     } else if (p->states > 1) {
         if constexpr (std::is_same<T, double>::value) {
             MixedPassArgs ma{};
@@ -1283,14 +1275,32 @@ void enqueue_multislice_iteration(cubo_ptycho_plan *p) {
     const double2 *shifted = p->shifted.as<double2>(), *props = p->props64.as<double2>();
     const Fft2Plan64 f = fft64(p);
     enqueue_shift_table<double>(p);
+    const RcGeometry rc = rc_geometry(p);
+    RcRows rows{};
+    rows.out_stride = n; rows.count = P; rows.layers = 1;
+    // the pointwise step of slice `sl` over its planes, in place
+    auto columns = [&](double2 *at, RcColumns c) {
+        c.planes = at; c.stride = n; c.count = P; c.layers = 1;
+        return launch_rc_columns(rc, c, s);
+    };
     if (p->rowcol64) {
-        for (int sl = 0; sl < L; sl++) {
-            const double2 *in = sl == 0 ? shifted : waves + (size_t)(sl - 1) * planes;
-            const bool last = sl == L - 1;
-            enqueue_rowcol(p, kPositionPass, in, sl == 0, 0, obj + (size_t)sl * plane, false,
-                           last ? rc_projection(p) : rc_propagation(p, sl, false),
-                           last ? chi : waves + (size_t)sl * planes, 0, 1);
-        }
+        // the spectrum of slice sl stands where the wave entering slice sl + 1 will, the last one's in chi
+        timed(p, kPositionPass, 2 * L + 1, [&] {
+            RcRows r = rows;
+            r.in = shifted; r.by_class = 1; r.object = obj; r.out = L > 1 ? waves : chi;
+            cudaError_t e = launch_rc_rows(rc, r, false, s);
+            r.by_class = 0;
+            for (int sl = 0; sl < L - 1 && e == cudaSuccess; sl++) {
+                double2 *at = waves + (size_t)sl * planes;
+                e = columns(at, rc_propagation(p, sl, false));
+                r.in = r.out = at; r.object = obj + (size_t)(sl + 1) * plane;
+                if (e == cudaSuccess) e = launch_rc_through(rc, r, sl + 2 < L ? at + planes : chi, s);
+            }
+            if (e == cudaSuccess) e = columns(chi, rc_projection(p));
+            r.out = chi;
+            if (e == cudaSuccess) e = launch_rc_rows(rc, r, true, s);
+            return e;
+        });
     } else {
     // forward (:503-515): exit_s = wave_s x O_s; wave_{s+1} = IFFT(FFT(exit_s) x prop_s / n)
     timed(p, kPositionPass, 6 * (L - 1) + 1, [&] {
@@ -1339,8 +1349,21 @@ void enqueue_multislice_iteration(cubo_ptycho_plan *p) {
         timed(p, kObjectGather, p->gather_groups > 1 ? 2 : 1, [&] { return gather_object<double>(p, ga); });
         if (sl == 0) break;
         if (p->rowcol64) {
-            enqueue_rowcol(p, kBackPropagation, chi, false, 0, obj + (size_t)sl * plane, true,
-                           rc_propagation(p, sl - 1, true), chi, 0, 1);
+            // chi conj(O_s) carried back through the gap: its spectrum stands in chi for the last slice, then, chi being
+            // read by the gathers, where the wave entering this slice was, which the gather above was the last to read
+            timed(p, kBackPropagation, sl == L - 1 ? 3 : 2, [&] {
+                RcRows r = rows;
+                r.conj_object = 1; r.object = obj + (size_t)sl * plane; r.in = r.out = chi;
+                cudaError_t e = cudaSuccess;
+                if (sl == L - 1) e = launch_rc_rows(rc, r, false, s);
+                double2 *at = sl == L - 1 ? chi : waves + (size_t)sl * planes;
+                if (e == cudaSuccess) e = columns(at, rc_propagation(p, sl - 1, true));
+                r.in = r.from = at; r.object = obj + (size_t)(sl - 1) * plane;
+                if (e == cudaSuccess)
+                    e = sl > 1 ? launch_rc_through(rc, r, waves + (size_t)(sl - 1) * planes, s)
+                               : launch_rc_rows(rc, r, true, s);
+                return e;
+            });
             continue;
         }
         timed(p, kBackPropagation, 6, [&] {

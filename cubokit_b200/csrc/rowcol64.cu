@@ -8,7 +8,7 @@
 //                  transforms.  The step is the modulus projection of one plane, the summed-intensity projection of the
 //                  mixed states' planes, a separable Fresnel propagator, or (no inverse, nothing written back) the normal
 //                  equations of position correction from three planes
-//   rows inverse   the inverse row transforms
+//   rows inverse   the inverse row transforms; multislice joins them with the next slice's forward rows (rc_through_kernel)
 //
 // Line transforms as in the any-size pass (anypass.cuh): in-place stages in registers, the first stage of a launch read from
 // and the last written to global memory, so a line of two stages crosses shared memory once each way.  128 has its
@@ -19,11 +19,11 @@
 // is quicker than the clustered launch that kept a 128 x 128 plane in two SMs and exchanged halves between them: there one
 // CTA an SM loaded, transformed and stored in turn, with HBM busy 15 % of the time; here two to six CTAs an SM overlap those.
 // 1,600 positions of 128 x 128, per iteration: four mixed states 3.5 -> 2.0 ms (their columns meet in one CTA, so the summed
-// projection needs no factor plane and no launch of its own), four slices forward 2.6 -> 2.1 and back 1.87 -> 1.55 ms; the
+// projection needs no factor plane and no launch of its own), four slices forward 2.6 -> 1.84 and back 1.87 -> 1.38 ms; the
 // three far fields and normal equations of 2,304 positions 2.7 -> 1.15 ms (the third field's columns end in the equations'
 // sums, which no field is written for).  Rows run at 4.6 TB/s, single columns at 4.5, limited by FP64 issue and LSU
 // wavefronts together.  Against the batched line transforms, which the generic variant, longer primes and sides up to 16 keep:
-// four slices of 980 positions of 96 x 96 58 -> 18.5 ms per seven iterations, two mixed states of 1,035 14.9 -> 4.7 per six.
+// four slices of 980 positions of 96 x 96 58 -> 17 ms per seven iterations, two mixed states of 1,035 14.9 -> 4.7 per six.
 #include <algorithm>
 #include <type_traits>
 
@@ -58,6 +58,8 @@ struct RcArgs {
     const double2 *object, *object_after; // null: no factor; object_after: position correction, whose layers are the object
     int conj_object;                      // before the update at the centre, after it a row and after it a column further
     double2 *out;                         // (columns: the planes in place)
+    double2 *next;                        // rows through: the next spectrum, laid out by position
+    const double2 *from;                  // rows inverse: the spectrum, by position (null: out itself)
     long long out_layer, out_stride;
     int out_first;
     int layers;
@@ -159,7 +161,8 @@ __global__ void __launch_bounds__(kRcThreads, 2) rc_rows_kernel(const __grid_con
     for (int i = threadIdx.x; i < L; i += kRcThreads) tw[i] = g.tw[i];
     for (int b = threadIdx.x; b < nb; b += kRcThreads) blocks_of[slot_frequency(g.line, b * l.last())] = (unsigned short)b;
     double2 *out = g.out + layer * g.out_layer + (long long)(p - g.out_first) * g.out_stride + (size_t)r0 * L;
-    const double2 *in = INV ? out : g.in + layer * g.in_layer +
+    const double2 *in = INV ? (g.from ? g.from + (long long)p * g.n + (size_t)r0 * L : out)
+                            : g.in + layer * g.in_layer +
                                         (size_t)(g.by_class ? g.scan.cls[p] : p) * g.n + (size_t)r0 * L;
     __syncthreads();
     if constexpr (!INV) {
@@ -242,6 +245,90 @@ __global__ void __launch_bounds__(kRcThreads, 2) rc_rows_kernel(const __grid_con
             }
         });
     }
+}
+
+// Multislice, between two slices: the inverse rows of one (whose wave or residual is written to out) and, while a row's samples
+// are in registers, their product with the object patch and the next slice's forward rows (written to next).  The last stage of
+// the one and the first of the other hold the same samples in the same thread.  `in` may be out or next.  A plane is read once
+// and written twice in place of two of each: four slices of 1,600 positions of 128 x 128, an iteration, forward 2.08 -> 1.84 ms,
+// back 1.55 -> 1.38.
+template <typename Line>
+__global__ void __launch_bounds__(kRcThreads, 2) rc_through_kernel(const __grid_constant__ RcArgs g) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double2 *D = reinterpret_cast<double2 *>(smem_raw);
+    const Line shape{g, nullptr};
+    const int L = shape.length(), nb = shape.blocks(), rl = shape.last() | 1, pitch = nb * rl;
+    double2 *tw = D + (size_t)shape.lines() * pitch;
+    unsigned short *blocks_of = reinterpret_cast<unsigned short *>(tw + L);
+    const Line l{g, blocks_of};
+    const int p = g.first + (int)(blockIdx.x / g.per), r0 = (int)(blockIdx.x % g.per) * l.lines();
+    const int rows = min(l.lines(), g.rows - r0);
+    for (int i = threadIdx.x; i < L; i += kRcThreads) tw[i] = g.tw[i];
+    for (int b = threadIdx.x; b < nb; b += kRcThreads) blocks_of[slot_frequency(g.line, b * l.last())] = (unsigned short)b;
+    const long long at = (long long)p * g.n + (size_t)r0 * L;
+    const double2 *in = g.in + at;
+    double2 *out = g.out + at, *next = g.next + at;
+    const int rr = g.scan.rr[p], cc = g.scan.cc[p];
+    __syncthreads();
+    l.inner_most([&](auto rc) {
+        constexpr int R = decltype(rc)::value;
+        for (int i = threadIdx.x; i < rows * nb; i += kRcThreads) {
+            const int row = l.by_blocks(i), K = i - row * nb;
+            const double2 *o = in + (size_t)row * L + K;
+            double2 x[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) x[r] = o[r * nb];
+            regdft::dft<double, true, R>(x);
+            double2 *y = D + row * pitch + l.base(K) * rl;
+#pragma unroll
+            for (int r = 0; r < R; r++) y[r] = x[r];
+        }
+    });
+    __syncthreads();
+    rows_between<true>(l, D, rows, pitch, tw);
+    l.outer([&](auto rc) {
+        constexpr int R = decltype(rc)::value;
+        const int sub = l.sub(), step = l.padded(sub);
+        for (int i = threadIdx.x; i < rows * sub; i += kRcThreads) {
+            const int row = l.by_sub(i), j = i - row * sub;
+            double2 *y = D + row * pitch + l.padded(j);
+            double2 x[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) x[r] = y[r * step];
+            twiddle<double, true, R>(x, j, 1, tw);
+            regdft::dft<double, true, R>(x);
+            double2 *o = out + (size_t)row * L + j;
+            const double2 *orow = g.object + (size_t)rc_wrap(rr + corner_offset(r0 + row, g.rows), g.object_rows) *
+                                                 g.object_columns;
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                o[r * sub] = x[r];
+                double2 f = orow[rc_wrap(cc + corner_offset(j + r * sub, L), g.object_columns)];
+                if (g.conj_object) f.y = -f.y;
+                x[r] = cmul(x[r], f);
+            }
+            regdft::dft<double, false, R>(x);
+            twiddle<double, false, R>(x, j, 1, tw);
+#pragma unroll
+            for (int r = 0; r < R; r++) y[r * step] = x[r];
+        }
+    });
+    __syncthreads();
+    rows_between<false>(l, D, rows, pitch, tw);
+    l.inner_most([&](auto rc) {
+        constexpr int R = decltype(rc)::value;
+        for (int i = threadIdx.x; i < rows * nb; i += kRcThreads) {
+            const int row = l.by_blocks(i), K = i - row * nb;
+            const double2 *y = D + row * pitch + l.base(K) * rl;
+            double2 x[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) x[r] = y[r];
+            regdft::dft<double, false, R>(x);
+            double2 *o = next + (size_t)row * L + K;
+#pragma unroll
+            for (int r = 0; r < R; r++) o[r * nb] = x[r];
+        }
+    });
 }
 
 // The columns of one position: plane y's sample e of column c at D[(y L + e) lines + c].
@@ -509,6 +596,7 @@ int rowcol64_parts(int rows, int columns, int layers) {
 cudaError_t configure_rowcol64() {
     const RcKernel kernels[] = {rc_rows_kernel<RunTimeLine, false>, rc_rows_kernel<RunTimeLine, true>,
                                 rc_rows_kernel<Row128, false>, rc_rows_kernel<Row128, true>,
+                                rc_through_kernel<RunTimeLine>, rc_through_kernel<Row128>,
                                 rc_columns_kernel<RunTimeLine, kRcProject>, rc_columns_kernel<RunTimeLine, kRcPropagate>,
                                 rc_columns_kernel<RunTimeLine, kRcMixed>, rc_columns_kernel<RunTimeLine, kRcSolve>,
                                 rc_columns_kernel<Column128, kRcProject>, rc_columns_kernel<Column128, kRcPropagate>,
@@ -526,7 +614,7 @@ cudaError_t launch_rc_rows(const RcGeometry &q, const RcRows &r, bool inverse, c
     size_t smem = 0;
     if (!rc_setup(&g, q.columns, q.rows, 1, false, &smem)) return cudaErrorInvalidValue;
     g.tw = q.tw_columns;
-    g.in = r.in; g.by_class = r.by_class; g.in_layer = r.in_layer;
+    g.in = r.in; g.by_class = r.by_class; g.in_layer = r.in_layer; g.from = r.from;
     g.object = r.object; g.object_after = r.object_after; g.conj_object = r.conj_object;
     g.out = r.out; g.out_layer = r.out_layer; g.out_stride = r.out_stride; g.out_first = r.out_first;
     const bool fixed = q.columns == 128;
@@ -534,6 +622,17 @@ cudaError_t launch_rc_rows(const RcGeometry &q, const RcRows &r, bool inverse, c
                                : (fixed ? rc_rows_kernel<Row128, false> : rc_rows_kernel<RunTimeLine, false>);
     g.layers = r.layers;
     return launch_rc(k, g, r.first, r.count, r.layers, kRcThreads, smem, s);
+}
+
+cudaError_t launch_rc_through(const RcGeometry &q, const RcRows &r, double2 *next, cudaStream_t s) {
+    if (r.count <= 0) return cudaSuccess;
+    RcArgs g = base_args(q);
+    size_t smem = 0;
+    if (!rc_setup(&g, q.columns, q.rows, 1, false, &smem)) return cudaErrorInvalidValue;
+    g.tw = q.tw_columns;
+    g.in = r.in; g.object = r.object; g.conj_object = r.conj_object; g.out = r.out; g.next = next;
+    return launch_rc(q.columns == 128 ? rc_through_kernel<Row128> : rc_through_kernel<RunTimeLine>, g, r.first, r.count, 1,
+                     kRcThreads, smem, s);
 }
 
 cudaError_t launch_rc_columns(const RcGeometry &q, const RcColumns &c, cudaStream_t s) {

@@ -65,3 +65,14 @@ def test_position_correction(rows, columns):
 def test_single_slice(rows, columns):
     s = _scene(rows, columns)
     _compare(s, lambda cb: dict(precision="fp64"), s["object"], s["probe"])
+
+
+@pytest.mark.parametrize("slices", [1, 2, 4, 5])
+@pytest.mark.parametrize("rows,columns", [(24, 36), (128, 40), (40, 288)])
+def test_multislice_depths(rows, columns, slices):
+    """No gap, one, and several (a wave's place is taken over by a spectrum once its gather has read it)."""
+    s = _scene(rows, columns)
+    obj = np.stack([s["object"] * np.exp(0.02j * i) for i in range(slices)])
+    ms = dict(slices=slices, slice_thicknesses=[20.0 + 5 * i for i in range(slices - 1)], wavelength=0.0197,
+              row_sampling=0.45, column_sampling=0.5)
+    _compare(s, lambda cb: dict(multislice=ms), obj, s["probe"])
