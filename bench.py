@@ -727,9 +727,9 @@ def run_positions(args, world, rank, local):
             "roofline": {"kernel": "position update (exit waves, FP64 far fields, 2x2 solves)", "bound": "hbm",
                          "achieved": corr_bytes / (corr_ms * 1e-3) / 1e9, "peak": hbm_peak, "unit": "GB/s",
                          "frac": corr_bytes / (corr_ms * 1e-3) / 1e9 / hbm_peak, "peak_kind": peak_kind,
-                         "launch_ms": corr_ms, "note": "three forward plane launches write each position's far "
-                                                       "fields, the 2x2 solves read them back; 20 bytes per pixel is "
-                                                       "the algorithmic floor",
+                         "launch_ms": corr_ms, "note": "row transforms of each position's three far fields, "
+                                                       "whose columns end in the 2x2 normal equations; 20 bytes per "
+                                                       "pixel is the algorithmic floor",
                          "traffic": None},
             "kernel_ms_per_iteration": per_kind, "moved_px_max": moved,
             "cpu_baseline": cpu, "e2e": None, "gpu_launches": launches, "clocks": clocks.summary()}), flush=True)
@@ -797,13 +797,13 @@ def run_mixed(args, world, rank, local):
             "config": {"workload": f"mixed: {P} positions ({args.scan}^2 raster), {DET}x{DET} detector, "
                                    f"{states} states, centre of mass + orthogonalisation",
                        "l2": "amplitudes 4.3 GB, residuals 69 GB: far larger than L2"},
-            "roofline": {"kernel": "mixed position pass (per state a forward plane launch, the summed-intensity "
-                                   "projection, per state an inverse plane launch; FP64)",
+            "roofline": {"kernel": "mixed position pass (rows of every state, columns with the summed-intensity "
+                                   "projection, inverse rows; FP64)",
                          "bound": "hbm", "achieved": pass_bytes / (pass_ms * 1e-3) / 1e9, "peak": hbm_peak,
                          "unit": "GB/s", "frac": pass_bytes / (pass_ms * 1e-3) / 1e9 / hbm_peak,
                          "peak_kind": peak_kind, "launch_ms": pass_ms,
-                         "note": "every state's far field is written, projected in place and read back (the "
-                                 "projection needs all states); the plane launches are latency-bound",
+                         "note": "every state's plane is read and written three times; the columns of all "
+                                 "states meet in one block, so the projection needs no launch of its own",
                          "traffic": None, "fft_equivalent_tflops": pass_flops / (pass_ms * 1e-3) / 1e12,
                          "frac_of_fp64_fma_peak": pass_flops / (pass_ms * 1e-3) / 1e12 / peaks["fp64_tflops"],
                          "cuda_core_peaks": peaks},
@@ -954,13 +954,13 @@ def run_multislice(args, world, rank, local):
                                    f"{slices} slices {thickness:g} A apart, 300 kV, centre of mass",
                        "l2": f"amplitudes {P * n * 4 / 1e9:.1f} GB, entering waves and residuals "
                              f"{P * n * 16 * slices / 1e9:.0f} GB: far larger than L2"},
-            "roofline": {"kernel": "multislice forward pass (one clustered plane launch per slice: patch product, "
-                                   "FP64 FFT, propagator or projection, inverse FFT)",
+            "roofline": {"kernel": "multislice forward pass (rows times the patch, columns with the propagator or "
+                                   "the projection, inverse rows joined with the next slice's; FP64)",
                          "bound": "hbm", "achieved": pass_bytes / (pass_ms * 1e-3) / 1e9, "peak": hbm_peak,
                          "unit": "GB/s", "frac": pass_bytes / (pass_ms * 1e-3) / 1e9 / hbm_peak,
                          "peak_kind": peak_kind, "launch_ms": pass_ms,
-                         "note": "latency-bound: one 512-thread CTA per SM holds half a plane in registers; its "
-                                 "load, transform and store phases do not overlap", "traffic": None,
+                         "note": "FP64 issue and LSU: a slice's plane is read twice and written three times",
+                         "traffic": None,
                          "fft_equivalent_tflops": pass_flops / (pass_ms * 1e-3) / 1e12,
                          "frac_of_fp64_fma_peak": pass_flops / (pass_ms * 1e-3) / 1e12 / peaks["fp64_tflops"],
                          "cuda_core_peaks": peaks},

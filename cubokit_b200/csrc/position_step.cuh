@@ -1,5 +1,5 @@
-// The arithmetic of one position's update (Ptychography.swift:411-472), shared by the solve kernel and the fused
-// 128 x 128 plane launch: the per-pixel terms of the 2 x 2 normal equations and the step with its limits.
+// The arithmetic of one position's update (Ptychography.swift:411-472), shared by the solve kernel and the
+// column launch that ends in the normal equations: the per-pixel terms of the 2 x 2 normal equations and the step with its limits.
 #pragma once
 
 #include <cuda_runtime.h>
