@@ -118,7 +118,7 @@ def measured_peaks():
 PASS_DRAM_BYTES_PER_POSITION = {"split_bf16": 748.1e6 / 4096, "fp32": None}
 
 
-def position_pass_roofline(head, stats, P, n, objects, ms_iter, peaks, fma):
+def position_pass_roofline(head, stats, timed, P, n, objects, ms_iter, peaks, fma):
     """The dominant kernel (the position pass) against the roofline that binds its algorithmic work.
 
     Algorithmic work per position: the amplitudes read once (4n bytes) and two n-point 2-D FFTs plus 40 flops per
@@ -126,8 +126,7 @@ def position_pass_roofline(head, stats, P, n, objects, ms_iter, peaks, fma):
     could use, so HBM binds: achieved = 4 n P / launch time, frac = achieved / measured HBM copy rate.  The executed
     split-BF16 tensor work (100.7 MFLOP per position of real 128 x 128 x 128 products) is reported beside it as a
     utilisation figure, not as the roofline."""
-    pass_ms, pass_launches = stats["position_pass"]
-    pass_s = pass_ms / max(pass_launches, 1) * 1e-3
+    pass_s = stats["position_pass"][0] / timed * 1e-3
     pass_bytes = P * 4 * n
     achieved = pass_bytes / pass_s / 1e9
     per_position = PASS_DRAM_BYTES_PER_POSITION.get(head)
@@ -1063,11 +1062,12 @@ def main():
         errors = plan.errors(args.warmup + args.steps)
         # per-kernel device time over separate iterations (events around every launch)
         plan.set_timing(True)
-        plan.enqueue(max(3, min(args.steps, 10)))
+        timed = max(3, min(args.steps, 10))
+        plan.enqueue(timed)
         stats = plan.kernel_stats()
         plan.set_timing(False)
         plan.close()
-        results[form] = dict(ms=ms, launches=launches, errors=errors, stats=stats, clocks=clocks.summary())
+        results[form] = dict(ms=ms, timed=timed, launches=launches, errors=errors, stats=stats, clocks=clocks.summary())
 
     head = forms[0]
     r = results[head]
@@ -1076,13 +1076,13 @@ def main():
     value = P * args.steps / (ms * 1e-3) * world
     peaks = measured_peaks()
     fma = fma_peaks(ctx)
-    roofline = position_pass_roofline(head, stats, P, n, objects, ms / args.steps, peaks, fma)
+    roofline = position_pass_roofline(head, stats, r["timed"], P, n, objects, ms / args.steps, peaks, fma)
     total_stat_ms = sum(v[0] for v in stats.values())
 
     fft_flops = P * (10 * n * math.log2(n) + 40 * n)
     forms_out = {}
     for form, fr in results.items():
-        pass_form_ms = fr["stats"]["position_pass"][0] / max(fr["stats"]["position_pass"][1], 1)
+        pass_form_ms = fr["stats"]["position_pass"][0] / fr["timed"]  # a pass may be several launches
         forms_out[form] = {"value": P * args.steps / (fr["ms"] * 1e-3) * world, "ms_per_step": fr["ms"] / args.steps,
                            "position_pass_ms": pass_form_ms, "error_last": float(fr["errors"][-1]),
                            "fft_equivalent_tflops": fft_flops / (pass_form_ms * 1e-3) / 1e12}
