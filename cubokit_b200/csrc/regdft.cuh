@@ -2,7 +2,7 @@
 //
 // Composite radices split once (R = A B, A-point DFTs, the twiddle W_R^{bc}, B-point DFTs); odd primes pair the samples
 // k and R - k, so an R-point DFT costs (R - 1)^2 / 2 real-by-complex multiply-adds.  Every constant is cos / sin of
-// 2 pi k / R evaluated at compile time in double and rounded once.  Forward is e^{-2 pi i}, both directions unnormalised.
+// 2 pi k / R evaluated at compile time and rounded to the nearest double (tests/test_regdft_constants.py).  Forward is e^{-2 pi i}, both directions unnormalised.
 #pragma once
 
 #include "common.cuh"
@@ -10,29 +10,63 @@
 namespace cubo {
 namespace regdft {
 
-// cos and sin of 2 pi k / n, 0 <= k < n, by their Taylor series on the first octant (compile time only).
-constexpr double taylor_cos(double x) {
-    double term = 1, sum = 1;
-    for (int i = 1; i < 14; i++) { term *= -x * x / ((2 * i - 1) * (2 * i)); sum += term; }
-    return sum;
+// cos and sin of 2 pi k / n, 0 <= k < n, rounded to the nearest double (compile time only): Taylor series on the first
+// octant in pairs of doubles (T. J. Dekker, "A floating-point technique for extending the available precision", Numer.
+// Math. 18, 1971), some 100 bits.  In plain double the sums' own roundings left half the constants of radix 8 and 16 one
+// unit off, and a constant that is short acts on every plane as the same small gain: with them the errors of four mixed states
+// of 128 x 128 were 1.4e-15 from 64 bits after four iterations, 3.4e-16 with these (objects 1.7e-16, 1.4e-16; four slices'
+// errors 1.0e-15, 3.4e-16).
+struct Pair {
+    double hi, lo;
+};
+constexpr Pair two_sum(double a, double b) {
+    const double s = a + b, t = s - a;
+    return Pair{s, (a - (s - t)) + (b - t)};
 }
-constexpr double taylor_sin(double x) {
-    double term = x, sum = x;
-    for (int i = 1; i < 14; i++) { term *= -x * x / ((2 * i) * (2 * i + 1)); sum += term; }
-    return sum;
+constexpr Pair two_product(double a, double b) {
+    constexpr double kSplit = 134217729.0;  // 2^27 + 1
+    const double ah = kSplit * a - (kSplit * a - a), al = a - ah, bh = kSplit * b - (kSplit * b - b), bl = b - bh;
+    const double p = a * b;
+    return Pair{p, ((ah * bh - p) + ah * bl + al * bh) + al * bl};
 }
-constexpr double kTwoPi = 6.283185307179586476925286766559;
+constexpr Pair add(Pair a, Pair b) {
+    const Pair s = two_sum(a.hi, b.hi);
+    return two_sum(s.hi, s.lo + (a.lo + b.lo));
+}
+constexpr Pair multiply(Pair a, Pair b) {
+    const Pair p = two_product(a.hi, b.hi);
+    return two_sum(p.hi, p.lo + (a.hi * b.lo + a.lo * b.hi));
+}
+constexpr Pair divide(Pair a, int d) {
+    const double q = a.hi / d;
+    const Pair p = two_product(q, (double)d);
+    return two_sum(q, (((a.hi - p.hi) - p.lo) + a.lo) / d);
+}
+// sum of (-1)^i x^(2 i + first) / (2 i + first)!, first = 0 (cosine) or 1 (sine)
+constexpr double taylor(Pair x, int first) {
+    const Pair square = multiply(x, x);
+    Pair term = first ? x : Pair{1, 0}, sum = term;
+    for (int i = 1; i < 16; i++) {
+        term = divide(multiply(term, Pair{-square.hi, -square.lo}), (2 * i - 1 + first) * (2 * i + first));
+        sum = add(sum, term);
+    }
+    return sum.hi;
+}
+// 2 pi k / n
+constexpr Pair angle(int k, int n) {
+    return divide(multiply(Pair{6.283185307179586, 2.4492935982947064e-16}, Pair{(double)k, 0}), n);
+}
 constexpr double turn_cos(int k, int n) {
     k %= n;
     if (2 * k > n) k = n - k;                              // cos(2 pi - a) = cos a
     if (4 * k > n) return -turn_cos(n - 2 * k, 2 * n);     // cos a = -cos(pi - a); the angle 2 pi (n - 2k) / (2n)
-    return 8 * k > n ? taylor_sin(kTwoPi * (n - 4 * k) / (4.0 * n)) : taylor_cos(kTwoPi * k / n);
+    return 8 * k > n ? taylor(angle(n - 4 * k, 4 * n), 1) : taylor(angle(k, n), 0);
 }
 constexpr double turn_sin(int k, int n) {
     k %= n;
     if (2 * k > n) return -turn_sin(n - k, n);
     if (4 * k > n) return turn_sin(n - 2 * k, 2 * n);      // sin a = sin(pi - a)
-    return 8 * k > n ? taylor_cos(kTwoPi * (n - 4 * k) / (4.0 * n)) : taylor_sin(kTwoPi * k / n);
+    return 8 * k > n ? taylor(angle(n - 4 * k, 4 * n), 0) : taylor(angle(k, n), 1);
 }
 template <int R>
 struct Turns {
