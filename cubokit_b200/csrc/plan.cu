@@ -17,12 +17,11 @@
 #include <mutex>
 #include <new>
 #include <string>
-#include <system_error>
-#include <thread>
 #include <vector>
 
 #include "../../include/cubo_ptycho.h"
 #include "engine.h"
+#include "host_ranges.h"
 
 using namespace cubo;
 
@@ -213,27 +212,6 @@ void *pinned_staging(cubo_ptycho_context *ctx, size_t bytes) {
 }
 
 namespace {
-
-// body(first, last) over `count` items in ranges of at least `grain` on up to eight host threads, the caller's among them
-// (a thread costs about 20 us to start; a complex value takes about 2 ns to convert on one).  body must not throw.
-template <typename F>
-void parallel_ranges(size_t count, size_t grain, const F &body) {
-    const size_t most = std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
-    const size_t parts = std::max<size_t>(1, std::min(most, count / grain));
-    std::vector<std::thread> threads;
-    size_t started = 1;
-    try {
-        threads.reserve(parts);
-        for (; started < parts; started++)
-            threads.emplace_back([&body, count, parts, part = started] {
-                body(count * part / parts, count * (part + 1) / parts);
-            });
-    } catch (const std::system_error &) {  // no more threads: the caller does the rest
-    }
-    body(0, count / parts);
-    for (size_t part = started; part < parts; part++) body(count * part / parts, count * (part + 1) / parts);
-    for (auto &t : threads) t.join();
-}
 
 constexpr size_t kConvertGrain = 1 << 18;  // values: half a millisecond on one thread
 
