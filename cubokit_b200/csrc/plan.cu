@@ -22,8 +22,19 @@
 #include "../../include/cubo_ptycho.h"
 #include "engine.h"
 #include "host_ranges.h"
+#include "host_staging.h"
 
 using namespace cubo;
+
+namespace {
+void *allocate_pinned(size_t bytes) {
+    void *ptr = nullptr;
+    if (cudaHostAlloc(&ptr, bytes, cudaHostAllocDefault) == cudaSuccess) return ptr;
+    cudaGetLastError();
+    return nullptr;
+}
+void free_pinned(void *ptr) { cudaFreeHost(ptr); }
+}  // namespace
 
 struct cubo_ptycho_context {
     int device = 0;
@@ -32,10 +43,7 @@ struct cubo_ptycho_context {
     bool timing = false;           // CUDA events around each preprocessing kernel launch
     double prepare_ms = 0.0;       // their device time, summed
     long long prepare_launches = 0;
-    // page-locked host staging for the object and probe transfers (grown on demand, freed with the context): copies
-    // from it run at full link speed and its pages are already mapped
-    void *pinned = nullptr;
-    size_t pinned_bytes = 0;
+    HostStaging staging{allocate_pinned, free_pinned};  // the object and probe transfers; freed with the context
 };
 
 namespace {
@@ -198,18 +206,6 @@ double bf16_to_double(uint16_t b) {
 }
 
 }  // namespace
-
-// The context's page-locked staging buffer of at least `bytes` (its contents are not kept when it grows).
-void *pinned_staging(cubo_ptycho_context *ctx, size_t bytes) {
-    if (ctx->pinned_bytes < bytes) {
-        if (ctx->pinned) cudaFreeHost(ctx->pinned);
-        ctx->pinned = nullptr;
-        ctx->pinned_bytes = 0;
-        check(cudaHostAlloc(&ctx->pinned, bytes, cudaHostAllocDefault), "cudaHostAlloc staging");
-        ctx->pinned_bytes = bytes;
-    }
-    return ctx->pinned;
-}
 
 namespace {
 
@@ -1550,7 +1546,6 @@ int cubo_ptycho_destroy(cubo_ptycho_context *ctx) {
         cudaStreamDestroy(ctx->stream);
     }
     BlockCache::get().context_destroyed(ctx->device);
-    if (ctx->pinned) cudaFreeHost(ctx->pinned);
     delete ctx;
     return CUBO_PTYCHO_OK;
 }
@@ -1905,19 +1900,17 @@ int set_state(cubo_ptycho_plan *p, const ComplexIn &object, const ComplexIn &pro
         const size_t object_values = (size_t)p->slices * p->objects;  // every slice, [slice][row][column]
         const size_t probe_values = (size_t)p->states * p->n;         // every probe state, [state][row][column]
         cudaStream_t s = p->ctx->stream;
-        // through the context's pinned staging buffer: the probe (complex128), then the object in the plan's type
         const size_t object_bytes = object_values * (p->fp64 ? sizeof(double2) : sizeof(float2));
-        uint8_t *stage = static_cast<uint8_t *>(pinned_staging(p->ctx, probe_values * sizeof(double2) + object_bytes));
-        uint8_t *object_stage = stage + probe_values * sizeof(double2);
-        const bool finite = p->fp64 ? convert_in(object, reinterpret_cast<double2 *>(object_stage), object_values)
-                                    : convert_in(object, reinterpret_cast<float2 *>(object_stage), object_values);
+        const StagedState stage(p->ctx->staging, probe_values, object_bytes);
+        const bool finite = p->fp64 ? convert_in(object, reinterpret_cast<double2 *>(stage.object), object_values)
+                                    : convert_in(object, reinterpret_cast<float2 *>(stage.object), object_values);
         if (!finite) fail(CUBO_PTYCHO_INVALID_INPUT, "object not finite");
-        if (!convert_in(probe, reinterpret_cast<double2 *>(stage), probe_values))
+        if (!convert_in(probe, reinterpret_cast<double2 *>(stage.probe), probe_values))
             fail(CUBO_PTYCHO_INVALID_INPUT, "probe not finite");
         p->tape_valid = false;
-        check(cudaMemcpyAsync(p->probe64.ptr, stage, probe_values * sizeof(double2), cudaMemcpyHostToDevice, s),
+        check(cudaMemcpyAsync(p->probe64.ptr, stage.probe, probe_values * sizeof(double2), cudaMemcpyHostToDevice, s),
               "upload probe");
-        check(cudaMemcpyAsync(p->object.ptr, object_stage, object_bytes, cudaMemcpyHostToDevice, s), "upload object");
+        check(cudaMemcpyAsync(p->object.ptr, stage.object, object_bytes, cudaMemcpyHostToDevice, s), "upload object");
         check(cudaStreamSynchronize(s), "sync");
         // the initial Fourier amplitude for fixProbeAperture (PtychographyConstraints.swift:79-83)
         if (p->params.fix_probe_aperture) {
@@ -1936,16 +1929,14 @@ int get_state(cubo_ptycho_plan *p, const ComplexOut &object, const ComplexOut &p
         const size_t probe_values = (size_t)p->states * p->n;
         const size_t object_values = (size_t)p->slices * p->objects;
         const size_t object_bytes = object_values * (p->fp64 ? sizeof(double2) : sizeof(float2));
-        uint8_t *stage = static_cast<uint8_t *>(pinned_staging(p->ctx, probe_values * sizeof(double2) + object_bytes));
-        const uint8_t *object_stage = stage + probe_values * sizeof(double2);
-        check(cudaMemcpyAsync(stage, p->probe64.ptr, probe_values * sizeof(double2), cudaMemcpyDeviceToHost, s),
+        const StagedState stage(p->ctx->staging, probe_values, object_bytes);
+        check(cudaMemcpyAsync(stage.probe, p->probe64.ptr, probe_values * sizeof(double2), cudaMemcpyDeviceToHost, s),
               "download probe");
-        check(cudaMemcpyAsync(stage + probe_values * sizeof(double2), p->object.ptr, object_bytes,
-                              cudaMemcpyDeviceToHost, s), "download object");
+        check(cudaMemcpyAsync(stage.object, p->object.ptr, object_bytes, cudaMemcpyDeviceToHost, s), "download object");
         check(cudaStreamSynchronize(s), "sync");
-        if (p->fp64) convert_out(reinterpret_cast<const double2 *>(object_stage), object_values, 1.0, object);
-        else convert_out(reinterpret_cast<const float2 *>(object_stage), object_values, 1.0, object);
-        convert_out(reinterpret_cast<const double2 *>(stage), probe_values, 1.0, probe);
+        if (p->fp64) convert_out(reinterpret_cast<const double2 *>(stage.object), object_values, 1.0, object);
+        else convert_out(reinterpret_cast<const float2 *>(stage.object), object_values, 1.0, object);
+        convert_out(reinterpret_cast<const double2 *>(stage.probe), probe_values, 1.0, probe);
     });
 }
 }  // namespace
@@ -2124,17 +2115,15 @@ void download_gradients(cubo_ptycho_plan *p, double scale, const ComplexOut &obj
                         double *loss) {
     cudaStream_t s = p->ctx->stream;
     const size_t probe_bytes = (size_t)p->n * sizeof(double2), object_bytes = (size_t)p->objects * sizeof(C2<T>);
-    uint8_t *stage = static_cast<uint8_t *>(pinned_staging(p->ctx, probe_bytes + object_bytes + sizeof(double)));
-    double *l = reinterpret_cast<double *>(stage + probe_bytes + object_bytes);
-    check(cudaMemcpyAsync(stage, p->grad_p64.ptr, probe_bytes, cudaMemcpyDeviceToHost, s), "download gradient");
-    check(cudaMemcpyAsync(stage + probe_bytes, p->grad_o.ptr, object_bytes, cudaMemcpyDeviceToHost, s),
-          "download gradient");
-    check(cudaMemcpyAsync(l, p->loss_slot.ptr, sizeof(double), cudaMemcpyDeviceToHost, s), "loss");
+    const StagedState stage(p->ctx->staging, (size_t)p->n, object_bytes);
+    check(cudaMemcpyAsync(stage.probe, p->grad_p64.ptr, probe_bytes, cudaMemcpyDeviceToHost, s), "download gradient");
+    check(cudaMemcpyAsync(stage.object, p->grad_o.ptr, object_bytes, cudaMemcpyDeviceToHost, s), "download gradient");
+    check(cudaMemcpyAsync(stage.value, p->loss_slot.ptr, sizeof(double), cudaMemcpyDeviceToHost, s), "loss");
     check(cudaStreamSynchronize(s), "sync");
     check_fault(p);
-    convert_out(reinterpret_cast<const C2<T> *>(stage + probe_bytes), (size_t)p->objects, scale, object);
-    convert_out(reinterpret_cast<const double2 *>(stage), (size_t)p->n, scale, probe);
-    if (loss) *loss = *l;
+    convert_out(reinterpret_cast<const C2<T> *>(stage.object), (size_t)p->objects, scale, object);
+    convert_out(reinterpret_cast<const double2 *>(stage.probe), (size_t)p->n, scale, probe);
+    if (loss) *loss = *stage.value;
 }
 
 int backward(cubo_ptycho_plan *p, int recompute, double *loss, const ComplexOut &object, const ComplexOut &probe) {
