@@ -143,7 +143,8 @@ constexpr int kTileW = 16, kTileH = 16;  // default object-gather tile (one pixe
 constexpr int kGatherThreads = kTileW * kTileH;
 
 // engine_kernels.cu
-template <typename T> cudaError_t launch_position_pass(const PositionPassArgs<T> &a, int shape, cudaStream_t s);
+template <typename T>
+cudaError_t launch_position_pass(const PositionPassArgs<T> &a, int shape, bool stockham, cudaStream_t s);
 // anypass.cu: the shared-memory position pass for any detector whose sides have no prime factor above 31 and whose plane
 // (with an odd pitch) fits one CTA; the pass of every such size without a compile-time plan.
 bool any_pass_applicable(int rows, int columns, bool fp64);

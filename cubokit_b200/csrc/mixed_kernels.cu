@@ -14,7 +14,6 @@
 #include <cfloat>
 
 #include "engine.h"
-#include "project.cuh"
 
 namespace cubo {
 
@@ -69,8 +68,15 @@ __global__ void __launch_bounds__(kProjectThreads) mixed_project_kernel(double2 
             const double2 f = dpsi[((size_t)s * count + p) * n + k];
             intensity += f.x * f.x + f.y * f.y;
         }
-        const double measured = (double)A[k];
-        const double factor = mixed_factor(intensity, measured, inv_n, zero_infinite != 0, err);
+        const double amplitude = sqrt(intensity), measured = (double)A[k];
+        double factor;
+        if (amplitude == 0.0) {
+            err += zero_infinite ? (double)INFINITY : measured * measured;
+            factor = 0.0;
+        } else {
+            err += (measured - amplitude) * (measured - amplitude);
+            factor = (measured / amplitude - 1.0) * inv_n;
+        }
         for (int s = 0; s < states; s++) {
             double2 *f = dpsi + ((size_t)s * count + p) * n + k;
             f->x *= factor;

@@ -284,6 +284,7 @@ struct cubo_ptycho_plan {
     int tile_w = kTileW, tile_h = kTileH;  // object-gather tile
     int probe_blocks = 0;
     bool fast = false;      // 128 x 128 FP32 register-resident position pass
+    bool stockham = false;  // the generic variant: no other shared-memory pass than position_pass_kernel
     bool bf16 = false;      // 128 x 128 split-BF16 tensor-core position pass
     bool global64 = false;  // FP64 position pass through global memory (the plane does not fit shared memory)
     bool global32 = false;  // FP32 position pass through global memory (global32.cu)
@@ -1012,7 +1013,7 @@ void enqueue_position_pass(cubo_ptycho_plan *p) {
             if (p->timing) p->kind_launches[kPositionPass] += count;
         }
     } else if (!p->grouped_pass) {
-        timed(p, kPositionPass, 1, [&] { return launch_position_pass<T>(pa, p->params.pass_shape, s); });
+        timed(p, kPositionPass, 1, [&] { return launch_position_pass<T>(pa, p->params.pass_shape, p->stockham, s); });
     }
 }
 
@@ -1695,8 +1696,8 @@ int create_plan(cubo_ptycho_context *ctx, const cubo_ptycho_problem *pr, const c
         check(configure_fft_lines(), "configure line transforms");
         p->bf16 = pp->form == CUBO_PTYCHO_FORM_SPLIT_BF16;
         if (p->bf16) check(configure_bf16(), "configure split-BF16 kernel");
-        p->fast = !p->fp64 && !p->bf16 && !p->global32 && pp->variant != CUBO_PTYCHO_VARIANT_GENERIC &&
-                  fast128_applicable(p->R, p->C);
+        p->stockham = pp->variant == CUBO_PTYCHO_VARIANT_GENERIC;
+        p->fast = !p->fp64 && !p->bf16 && !p->global32 && !p->stockham && fast128_applicable(p->R, p->C);
         if (p->fast) check(configure_fast128(), "configure 128 x 128 kernel");
         check(cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, ctx->device), "attribute");
         if (p->bf16 || p->fast) {
@@ -2313,7 +2314,7 @@ void build_groups(cubo_ptycho_batch *b) {
         if (p->fp64) ensure_dpsi<double>(p);
         else ensure_dpsi<float>(p);
         const bool generic_pass = p->fp64 ? !p->global64 : !p->fast && !p->bf16 && !p->global32;
-        if (generic_pass && position_pass_groupable(p->R, p->C, p->fp64)) {
+        if (generic_pass && !p->stockham && position_pass_groupable(p->R, p->C, p->fp64)) {
             add(0, p, p->R, p->params.pass_shape, p->P);
             p->grouped_pass = true;
         }

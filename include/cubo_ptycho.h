@@ -103,9 +103,9 @@ typedef struct {
     cubo_ptycho_progress_fn progress;
     void *progress_user;
     /* Kernel choice: CUBO_PTYCHO_VARIANT_AUTO picks the specialised kernel for the detector size when there is one;
-     * CUBO_PTYCHO_VARIANT_GENERIC forces the any-size transforms (for cross-checks): the shared-memory one, and for
-     * FP64 planes larger than one CTA the batched line transform through global memory instead of the row and column
-     * launches;
+     * CUBO_PTYCHO_VARIANT_GENERIC forces the Stockham transforms (for cross-checks; no code shared with the
+     * specialised kernels): the shared-memory pass, and for FP64 planes larger than one CTA the batched line transform
+     * through global memory instead of the row and column launches;
      * CUBO_PTYCHO_VARIANT_GLOBAL (FP64 and FP32 forms) forces the position pass through global memory that detectors
      * too large for one CTA's plane use (FP64: above 12,288 pixels; FP32: above 16,384, sides up to 4096) (for
      * cross-checks). */
