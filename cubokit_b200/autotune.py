@@ -5,19 +5,23 @@ candidate, a warm-up iteration, then the kernel's device time over a few iterati
 statistics.  `tune` picks the object-gather tile (32 x 8, 16 x 16, 64 x 4 pixels, along the residual's contiguous
 axis); `tune_pass` the CTA shape of the shared-memory position pass at the detectors it runs with a compile-time radix
 plan or the default FP32 kernel (64 x 64 and 96 x 96).  The fastest candidate is cached in a JSON file keyed by
-(what, detector, object, positions, form, GPU name), so the timing runs once per shape per machine.  Neither choice
+(what, detector, object, positions, form, GPU name), so the timing runs once per shape per machine, and again with
+another build of the library, whose kernels an earlier choice says nothing about.  Neither choice
 changes the object: every object pixel sums the same positions in the same order whatever the tile, and every
 butterfly computes the same values whatever the shared-memory CTA shape; the default FP32 kernel agrees with
 those to FP32 round-off.
 """
 from __future__ import annotations
 
+import functools
+import hashlib
 import json
 import os
 from pathlib import Path
 
 import numpy as np
 
+from . import _lib
 from .ptycho import Plan, context
 
 CANDIDATES = (1, 2, 3)  # 32 x 8, 16 x 16, 64 x 4
@@ -59,6 +63,12 @@ def device_name(device=0):
         return "cuda"
 
 
+@functools.lru_cache(maxsize=1)
+def library_id() -> str:
+    """What the loaded library is: a digest of its file."""
+    return hashlib.sha256(_lib.LIB_PATH.read_bytes()).hexdigest()[:16]
+
+
 def _time(amplitudes, positions, obj, probe, precision, iterations, device, kernel, option, candidates, names):
     ctx = context(device)
     timings = {}
@@ -80,13 +90,13 @@ def _tuned(what, amplitudes, positions, obj, probe, precision, iterations, devic
     probe = np.asarray(probe)
     k = what + "|" + key(probe.shape, obj.shape, len(positions), precision, device_name(device))
     table = _load() if use_cache else {}
-    if k in table:
+    if k in table and table[k].get("library") == library_id():
         return table[k]["choice"], table[k]["ms"]
     best, timings = _time(amplitudes, positions, obj, probe, precision, iterations, device, kernel, option, candidates,
                           names)
     if use_cache:
         table = _load()
-        table[k] = {"choice": best, "ms": timings}
+        table[k] = {"choice": best, "ms": timings, "library": library_id()}
         _store(table)
     return best, timings
 
