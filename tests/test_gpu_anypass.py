@@ -47,3 +47,18 @@ def test_fp64_against_the_oracles(rows, columns):
     assert np.max(np.abs(r.probe - p)) <= 1e-12 + 4 * np.max(np.abs(pn - p))
     assert np.allclose(r.errors, e, rtol=1e-9, atol=0)
     assert np.array_equal(r.object, runs[1].object) and np.array_equal(r.errors, runs[1].errors)
+
+
+@pytest.mark.parametrize("rows,columns", SIZES)
+def test_fp32_errors_and_bits(rows, columns):
+    """The squared residual, summed over CTAs of 128 to 1024 threads: with far fields off by d of the amplitudes' size it is
+    off by at most 2 d sqrt(e) for a residual of e (both over the amplitudes' energy), d = 5e-7 for FP32 transforms of up to
+    16,384 samples.  Twice the same bits."""
+    import cubokit_b200 as cb
+    s = scenes.raster_scene(scan=4, step=3, seed=5, shape=(rows, columns))
+    args = (s["amplitudes"].astype(np.float32), s["positions"], s["object"], s["probe"])
+    e = c_oracle.reconstruct(*args, iterations=3)[2]
+    first, second = (cb.SingleslicePtychography.reconstruct(*args, iterations=3) for _ in range(2))
+    assert np.all(np.abs(first.errors - e) <= 1e-6 * np.sqrt(e))
+    assert np.array_equal(first.errors, second.errors) and np.array_equal(first.object, second.object)
+    assert np.array_equal(first.probe, second.probe)
