@@ -181,7 +181,7 @@ template <typename T> int probe_gather_resident_ctas();  // CTAs of the probe ga
 template <typename T>
 cudaError_t launch_probe_reduce(const C2<T> *partial_grad, const T *partial_weight, int groups, int n,
                                 double2 *grad, double *weight, double *block_max, cudaStream_t s);
-int probe_reduce_blocks(int n);  // entries of block_max
+int probe_reduce_blocks(int n, int groups);  // entries of block_max
 cudaError_t launch_maxima(const double *values, int arrays, long long stride, long long count, double *out,
                           const double *last, long long last_count, double *out_last, cudaStream_t s);
 // The maximum of count values (float or double) into *out, one CTA in a fixed order.

@@ -517,15 +517,38 @@ __global__ void __launch_bounds__(kProbeThreads) probe_gather_grouped_kernel(con
     probe_gather_body<T>(a, v % blocks, v / blocks);
 }
 
-// The groups' probe sums in FP64: 32 pixels a CTA, warp w takes the w-th eighth of the groups in order, then the eighths
-// are added in order.  (One thread a pixel over every group left 16 to 64 CTAs walking up to 148 partials: 62 us for 128 x
-// 128, 13 us now.)
-constexpr int kReducePixels = 32, kReduceSlices = 8;
-template <typename T>
+// The groups' probe sums in FP64, 256 / SLICES pixels a CTA.  SLICES = 8: warp w takes the w-th eighth of the groups in
+// order, then the eighths are added in order.  SLICES = 1: a thread a pixel over every group.
+//
+// A detector of few pixels has many groups, and a thread a pixel would leave 16 to 64 CTAs walking up to 148 partials (128 x
+// 128 62 us, in eighths 13).  One of many pixels has few, and most of the eighths would be empty: with one group 4096 x 4096
+// takes 129 us so and 535 in eighths, 1024 x 1024 13 and 38, with three 256 x 256 7 and 9; with six (192 x 192) both take 7,
+// with eight (160 x 160) 9 and 7.  The maximum over the CTAs follows (4096 x 4096 13 us, 52).  Up to eight groups the sums have
+// the same bits in either form.
+constexpr int kReduceSlices = 8;
+constexpr int probe_reduce_slices(int groups) { return groups <= 6 ? 1 : kReduceSlices; }
+template <typename T, int SLICES>
 __global__ void __launch_bounds__(256) probe_reduce_kernel(const C2<T> *pg, const T *pw, int groups, int n,
                                                            double2 *grad, double *weight, double *block_max_out) {
-    __shared__ double sums[3][kReduceSlices][kReducePixels];
-    const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5, k = blockIdx.x * kReducePixels + lane;
+    if constexpr (SLICES == 1) {
+        __shared__ double scratch[32];
+        const int k = blockIdx.x * 256 + threadIdx.x;
+        double gx = 0, gy = 0, w = 0;
+        if (k < n) {
+            for (int g = 0; g < groups; g++) {
+                const C2<T> v = pg[(size_t)g * n + k];
+                gx += (double)v.x; gy += (double)v.y; w += (double)pw[(size_t)g * n + k];
+            }
+            grad[k] = make_double2(gx, gy);
+            weight[k] = w;
+        }
+        const double m = block_max<256>(k < n ? w : -DBL_MAX, scratch);
+        if (threadIdx.x == 0) block_max_out[blockIdx.x] = m;
+        return;
+    }
+    static_assert(SLICES == 1 || SLICES == 8, "one warp a slice");
+    __shared__ double sums[3][kReduceSlices][32];
+    const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5, k = blockIdx.x * 32 + lane;
     double gx = 0, gy = 0, w = 0;
     if (k < n) {
         const int end = groups * (slice + 1) / kReduceSlices;
@@ -946,11 +969,15 @@ int probe_gather_resident_ctas() {
 template <typename T>
 cudaError_t launch_probe_reduce(const C2<T> *pg, const T *pw, int groups, int n, double2 *grad, double *weight,
                                 double *block_max_out, cudaStream_t s) {
-    probe_reduce_kernel<T><<<probe_reduce_blocks(n), 256, 0, s>>>(pg, pw, groups, n, grad, weight, block_max_out);
+    auto kernel = probe_reduce_slices(groups) == 1 ? probe_reduce_kernel<T, 1> : probe_reduce_kernel<T, kReduceSlices>;
+    kernel<<<probe_reduce_blocks(n, groups), 256, 0, s>>>(pg, pw, groups, n, grad, weight, block_max_out);
     return cudaGetLastError();
 }
 
-int probe_reduce_blocks(int n) { return (n + kReducePixels - 1) / kReducePixels; }
+int probe_reduce_blocks(int n, int groups) {
+    const int pixels = 256 / probe_reduce_slices(groups);
+    return (n + pixels - 1) / pixels;
+}
 
 cudaError_t launch_maxima(const double *values, int arrays, long long stride, long long count, double *out,
                           const double *last, long long last_count, double *out_last, cudaStream_t s) {

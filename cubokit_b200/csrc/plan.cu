@@ -732,7 +732,7 @@ void build_plan(cubo_ptycho_plan *p, const cubo_ptycho_problem *pr) {
     check(p->partial_weight.alloc((size_t)p->groups * n * sizeof(T)), "cudaMalloc");
     check(p->grad_p64.alloc((size_t)p->states * n * sizeof(double2)), "cudaMalloc");
     check(p->weight_p64.alloc((size_t)n * sizeof(double)), "cudaMalloc");
-    p->probe_blocks = probe_reduce_blocks(n);
+    p->probe_blocks = probe_reduce_blocks(n, p->groups);
     check(p->probe_block_max.alloc((size_t)p->probe_blocks * sizeof(double)), "cudaMalloc");
     check(p->maxes.alloc(4 * sizeof(double)), "cudaMalloc");
     check(p->error_scratch.alloc((size_t)error_reduce_scratch() * sizeof(double)), "cudaMalloc");
