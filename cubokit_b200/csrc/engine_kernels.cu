@@ -219,13 +219,18 @@ __device__ __forceinline__ int lower_bound_index(const int *list, int lo, int hi
     return lo;
 }
 
-template <typename T, bool MIXED>
+// GROUPS: one group a tile or several, in instances of their own too (the batch's launch, whose items have either, tells them at
+// run time): what tells them apart took registers from the FP64 loads in flight (64 positions of 1024 x 1024, one group, 0.220 ms
+// with it, 0.211 without; FP32, several groups, 3,600 positions of 128 x 128 0.162 and 0.152).
+enum { kOneGroup, kSeveralGroups, kAnyGroups };
+template <typename T, bool MIXED, int GROUPS>
 __device__ __forceinline__ void object_gather_body(const ObjectGatherArgs<T> &a, int unit) {
     __shared__ int s_p[kGatherChunk], s_cls[kGatherChunk];
     __shared__ int s_off[kGatherChunk][kMaxTileSide + kGatherThreads / kMaxTileSide + 4];  // rows, then columns
     __shared__ double scratch[32];
     const int part = a.band_tiles ? a.band_tiles[unit] : unit;  // one group of a tile's candidates
-    const int tile = part / a.groups, group = part - tile * a.groups;
+    const bool split = GROUPS == kSeveralGroups || (GROUPS == kAnyGroups && a.groups > 1);
+    const int tile = GROUPS == kOneGroup ? part : part / a.groups, group = GROUPS == kOneGroup ? 0 : part - tile * a.groups;
     const int tx = tile % a.tiles_x, ty = tile / a.tiles_x;
     const int x0 = tx * a.tile_w, y0 = ty * a.tile_h;
     // consecutive threads take consecutive object columns, hence consecutive addresses of each [row][column] residual
@@ -236,8 +241,8 @@ __device__ __forceinline__ void object_gather_body(const ObjectGatherArgs<T> &a,
     C2<T> g = mk<T>(0, 0);
     T w = 0;
     // where this group's sums go: with several groups into its share of the partials, which object_combine_kernel adds
-    C2<T> *sum_grad = a.groups > 1 ? a.part_grad : a.grad;
-    T *sum_weight = a.groups > 1 ? a.part_weight : a.weight;
+    C2<T> *sum_grad = split ? a.part_grad : a.grad;
+    T *sum_weight = split ? a.part_weight : a.weight;
     const size_t j = ((size_t)group * a.object_rows + y) * a.object_columns + x;
     const int list_begin = a.tile_start[part], list_end = a.tile_start[part + 1];
     int begin = list_begin, end = list_end;
@@ -334,14 +339,14 @@ __device__ __forceinline__ void object_gather_body(const ObjectGatherArgs<T> &a,
         sum_grad[j] = g;
         sum_weight[j] = w;
     }
-    if (end != list_end || a.groups > 1) return;  // a later band or another group still adds (uniform over the block)
+    if (end != list_end || split) return;  // a later band or another group still adds (uniform over the block)
     const double m = block_max<kGatherThreads>(inside ? (double)w : -DBL_MAX, scratch);
     if (threadIdx.x == 0) a.tile_max[tile] = m;
 }
 
-template <typename T, bool MIXED>
+template <typename T, bool MIXED, int GROUPS>
 __global__ void __launch_bounds__(kGatherThreads) object_gather_kernel(ObjectGatherArgs<T> a) {
-    object_gather_body<T, MIXED>(a, blockIdx.x);
+    object_gather_body<T, MIXED, GROUPS>(a, blockIdx.x);
 }
 
 // The groups' object sums added in order, and each block's maximum of the weights.
@@ -375,7 +380,7 @@ __global__ void __launch_bounds__(kGatherThreads) object_gather_grouped_kernel(c
     const int u = blockIdx.x;
     const int it = group_item(prefix, items, u);
     const ObjectGatherArgs<T> a = args[it];
-    object_gather_body<T, false>(a, u - prefix[it]);
+    object_gather_body<T, false, kAnyGroups>(a, u - prefix[it]);
 }
 
 // Grouped combine: every item's blocks of 256 object pixels, one CTA per unit.
@@ -908,11 +913,14 @@ template <typename T>
 cudaError_t launch_object_gather(const ObjectGatherArgs<T> &a, int parts, cudaStream_t s) {
     if constexpr (std::is_same<T, double>::value) {
         if (a.states > 1) {  // the mixed-state form exists in FP64 only
-            object_gather_kernel<T, true><<<parts, kGatherThreads, 0, s>>>(a);
+            auto kernel = a.groups > 1 ? object_gather_kernel<T, true, kSeveralGroups>
+                                       : object_gather_kernel<T, true, kOneGroup>;
+            kernel<<<parts, kGatherThreads, 0, s>>>(a);
             return cudaGetLastError();
         }
     }
-    object_gather_kernel<T, false><<<parts, kGatherThreads, 0, s>>>(a);
+    auto kernel = a.groups > 1 ? object_gather_kernel<T, false, kSeveralGroups> : object_gather_kernel<T, false, kOneGroup>;
+    kernel<<<parts, kGatherThreads, 0, s>>>(a);
     return cudaGetLastError();
 }
 
