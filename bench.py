@@ -648,11 +648,11 @@ def run_preprocess(args, world, rank, local):
             "dtype": "f64 (f32 in and out)", "data": "synthetic",
             "config": {"workload": f"preprocess: {count} patterns of {DET}x{DET}, cubic spline, uniform origin "
                                    f"{origins}", "l2": "cube and amplitudes (4.3 GB each) far larger than L2"},
-            "roofline": {"kernel": "prepare_kernel<cubic, 128, 128>", "bound": "hbm",
+            "roofline": {"kernel": "prepare_spline_kernel<128, 128>", "bound": "hbm",
                          "achieved": bytes_step / (launch_ms * 1e-3) / 1e9, "peak": hbm_peak, "unit": "GB/s",
                          "frac": bytes_step / (launch_ms * 1e-3) / 1e9 / hbm_peak, "peak_kind": peak_kind,
                          "launch_ms": launch_ms, "launches": kernel_launches,
-                         "note": "instruction-issue bound (FP64 prefilter and taps), not HBM-bound",
+                         "note": "chains of dependent FP64 operations (prefilter and taps) at 16 warps an SM, not HBM-bound",
                          "traffic": None},
             "mean_intensity": out.mean_intensity, "clipped_mean_intensity": out.clipped_mean_intensity,
             "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": 3 * args.steps, "clocks": clocks.summary()}),
@@ -958,7 +958,7 @@ def run_multislice(args, world, rank, local):
                          "bound": "hbm", "achieved": pass_bytes / (pass_ms * 1e-3) / 1e9, "peak": hbm_peak,
                          "unit": "GB/s", "frac": pass_bytes / (pass_ms * 1e-3) / 1e9 / hbm_peak,
                          "peak_kind": peak_kind, "launch_ms": pass_ms,
-                         "note": "FP64 issue and LSU: a slice's plane is read twice and written three times",
+                         "note": "a slice's plane is read twice and written three times; no unit full (FP64 pipe 19 to 42 %)",
                          "traffic": None,
                          "fft_equivalent_tflops": pass_flops / (pass_ms * 1e-3) / 1e12,
                          "frac_of_fp64_fma_peak": pass_flops / (pass_ms * 1e-3) / 1e12 / peaks["fp64_tflops"],
@@ -974,7 +974,7 @@ def main():
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--form", default="both", choices=["both", "all", "fp32", "split_bf16"],
-                    help="both: split-BF16 (the headline) and FP32 measured on the same data; all: also the any-size "
+                    help="both: split-BF16 (the headline) and FP32 measured on the same data; all: also the generic "
                          "FP32 transform (fp32_generic) and the FP64 form")
     ap.add_argument("--no-e2e", action="store_true")
     ap.add_argument("--no-cpu", action="store_true")
@@ -1041,7 +1041,7 @@ def main():
         args.form, [args.form])
     results = {}
     for form in forms:
-        # fp32_generic: the FP32 form through the any-size shared-memory transform instead of the 128 x 128 kernel
+        # fp32_generic: the FP32 form through the generic variant's Stockham transform instead of the 128 x 128 kernel
         plan = cb.Plan(ds.amplitudes, ds.positions, ds.object_start.shape, ds.probe.shape, ctx=ctx, step_size=0.5,
                        precision="fp32" if form == "fp32_generic" else form,
                        variant="generic" if form == "fp32_generic" else "auto")

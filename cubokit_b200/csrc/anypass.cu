@@ -31,7 +31,7 @@ void (*any_kernel(bool wide_radices))(AnyPassArgs<T>) {
 
 // Threads per CTA by how many CTAs' planes fit one SM (the registers allow 1024 FP32 and 512 FP64 threads there): the SM
 // full, but no more than 128 threads for planes of a few thousand pixels, whose stages hold only n / 8 butterflies.
-// Measured at a 60^2 scan, ms per pass: FP32 80 x 80 (4 fit) 0.246 at 256 threads, 0.294 at 512, 0.284 at 128; 48 x 48
+// Measured at a 60^2 scan, before the projection's present form, ms per pass: FP32 80 x 80 (4 fit) 0.246 at 256 threads, 0.294 at 512, 0.284 at 128; 48 x 48
 // (11 fit) 0.097 at 128, 0.116 at 256; 120 x 112 (2 fit) 0.538 at 512, 0.596 at 256; 128 x 128 at a 64^2 scan (1 fits)
 // 0.794 at 1024, 0.866 at 512.  FP64 96 x 100 (1 fits) 1.00 at 512, 1.17 at 256; 60 x 60 (3 fit) 0.311 at 256, 0.342 at
 // 512; 40 x 40 (8 fit) 0.130 at 128, 0.141 at 256.

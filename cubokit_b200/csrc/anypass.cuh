@@ -19,9 +19,10 @@
 //    row, as global memory wants it.
 //  * Index divisions are multiplications by reciprocals made on the host.
 //
-// Bound by instruction issue and shared memory together (in the FP64 form by the FP64 pipe too), not by HBM.  Against the
-// run-time Stockham plan that served these sizes before (one 512-thread CTA per SM, its per-stage arrays in local memory,
-// a run-time modulo per twiddle), 3,180 positions of 120 x 112: 5.75 -> 0.47 ms per FP32 pass, 7 -> 90 Gpixel/s.
+// Bound by shared-memory wavefronts and issue together (FP32 120 x 112: 70 and 56 %; FP64 100 x 90, one CTA an SM: 56 and 35 %,
+// FP64 pipe 36 %), not by HBM.  Against the run-time Stockham plan (one 512-thread CTA per SM, its per-stage arrays in local
+// memory, a run-time modulo per twiddle), 3,180 positions of 120 x 112: 5.76 -> 0.39 ms per FP32 pass, 7 -> 110 Gpixel/s;
+// 3,600 of 100 x 100 in FP64 3.21 -> 0.70.
 #pragma once
 
 #include "engine.h"

@@ -25,7 +25,7 @@
 //    partial; a fixed-order FP64 reduction over the 148 partials follows.  This replaces a second pass over dpsi (0.35
 //    ms at 16,384 positions, against 0.19 ms here).
 //
-// Bound by instruction issue (0.6 of the slots) and the LSU pipe (0.6 of its wavefronts) together, HBM at 15%.  16,384
+// Bound by the LSU pipe (0.76 of its wavefronts) and instruction issue (0.59 of the slots) together, HBM at 20 %.  16,384
 // positions take 1.79 ms (150 Gpixel/s); before, 2.81 ms: 512 threads of 128 registers, each line pass a register-resident
 // four-step transform with an exchange in a padded tile and four CTA barriers a position (1.95 ms without the probe
 // gradient in this form against 2.30 with a CTA barrier at every stage, 2.45 without the fused ends).

@@ -341,7 +341,7 @@ cudaError_t launch_position_pass_global32(const PositionPassArgs<float> &a, int 
     };
     G32Args gr = args(pr, per_r), gc = args(pc, per_c);
     // Batches of positions whose CTAs fit one grid dimension.  (Batches small enough to stay in L2 between their launches,
-    // 19 to 111 MB of residuals, measured slower: 2.95 to 4.29 ms against 2.51 at 4,096 positions of 256 x 256; the gaps and
+    // 19 to 111 MB of residuals, measured slower, before the projection's present form: 2.95 to 4.29 ms against 2.51 at 4,096 positions of 256 x 256; the gaps and
     // part waves of 3 launches a batch cost more than the HBM traffic they save.)
     const int chunk = (int)std::max<long long>(1, (1LL << 30) / std::max(per_r, per_c));
     int count = 0;

@@ -18,10 +18,12 @@
 // which keeps both its stages free of bank conflicts.  128, 192 and 256 have their geometry fixed at compile time.  Lines
 // with a prime factor above 31 take the direct DFT (g32_rows_direct, g32_columns_direct).
 //
-// Bound by HBM: 52 bytes a pixel over the three launches, 106 Gpixel/s at 256 x 256 = 0.84 of the measured copy rate.  The
-// Stockham stages before (lines staged whole, two barriers a stage; a run-time plan that spilled beyond four lengths, line
-// counts that had to divide the side) took 4.27 ms per pass of 4,096 positions of 256 x 256, now 2.51; 128 x 225 4.72 ->
-// 0.87 (2,500 positions), 160 x 200 3.89 -> 0.81, 128 x 248 22.1 -> 0.96 (1,600), 96 x 211 5.83 -> 2.47 (400).
+// 44 bytes a pixel cross HBM over the three launches (the shifted probe and the object come from L2), 2.24 ms per pass of 4,096
+// positions of 256 x 256 = 0.80 of the measured copy rate (120 Gpixel/s).  The exit wave's rows are bound by LSU wavefronts (78 %
+// of the pipe), the columns by issue (71 %) beside HBM (60), the inverse rows by HBM (79).  The Stockham stages before (lines
+// staged whole, two barriers a stage; a run-time plan that spilled beyond four lengths, line counts that had to divide the
+// side) took 4.08 ms; 128 x 225 4.59 -> 0.80 (2,500 positions), 160 x 200 5.86 -> 1.13 (2,500), 128 x 248 22.1 -> 0.91 (1,600), 96 x
+// 211 5.78 -> 2.45 (400).
 #pragma once
 
 #include "anypass.cuh"

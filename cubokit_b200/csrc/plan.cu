@@ -49,7 +49,6 @@ struct cubo_ptycho_context {
 namespace {
 
 constexpr double kPi = 3.14159265358979323846;
-constexpr int kSide128 = 128;
 
 // --------------------------------------------------------------------------------------------- device buffers
 
@@ -340,7 +339,7 @@ struct cubo_ptycho_plan {
     DeviceBuffer positions64, initial64, object_before, far64, position_bad, fractions64;
     DeviceBuffer gram64, mixing64, ortho64;
     DeviceBuffer waves64, props64, ident, slice_max;  // multislice: entering waves, propagators, identity classes
-    DeviceBuffer prop_factors64;  // multislice, 128 x 128 planes: per gap the row and the column factor (128 + 128)
+    DeviceBuffer prop_factors64;  // multislice by row and column launches: per gap the row and the column factors (R + C)
     DeviceBuffer tile_counts;          // position correction: candidate counts per tile, rebuilt on the device
     DeviceBuffer band_tiles, dpsi_band;  // banded iterations: tiles per band, the residuals of one band
     DeviceBuffer shard_loss, shard_counter;  // sharded iterations: this plan's summed squared error, its reduce counter

@@ -469,9 +469,10 @@ __host__ __device__ __forceinline__ int spline_plane(int rows, int columns) {
 // the registers of the threads that hold its segments (the shift is one number for a pattern, so the taps of a segment are
 // its own coefficients and three of the next), rows first, then columns, whose results leave as they are.  A warp holds whole
 // lines, so segments exchange by shuffles: two block barriers a pattern in place of seven, one store and one load of shared
-// memory a value in place of two and seven.  Bound by FP64 and issue: 16,384 patterns of 128 x 128 1.375 -> 1.29 ms,
-// 12,000 of 112 x 128 1.41 -> 1.03, of 96 x 96 1.08 -> 0.91 and of 64 x 64, several CTAs an SM, 0.75 -> 0.30 (every size below
-// the limit was quicker this way; 1024 threads of 64 registers spilled: 1.55 ms at 128 x 128).
+// memory a value in place of two and seven.  Bound by the chains of dependent FP64 operations at 16 warps an SM (issue 53 %, FP64
+// pipe 30 %, shared memory 44 %): 16,384 patterns of 128 x 128 1.375 -> 1.29 ms, 12,000 of 112 x 128 1.41 -> 1.03, of 96 x 96
+// 1.08 -> 0.91 and of 64 x 64, several CTAs an SM, 0.75 -> 0.30 (no size from 16 x 16 to 512 x 16 and 16 x 512 below the limit was
+// slower by more than 1 %; 1024 threads of 64 registers spilled: 1.55 ms at 128 x 128).
 // While the columns are computed, the next pattern is copied in, its 16-byte units swizzled for the rows' loads.
 template <int kRows, int kColumns>
 __global__ void __launch_bounds__(kSplineThreads) prepare_spline_kernel(const float *cube, int count, int rows_arg,

@@ -21,8 +21,9 @@
 // 1,600 positions of 128 x 128, per iteration: four mixed states 3.5 -> 2.0 ms (their columns meet in one CTA, so the summed
 // projection needs no factor plane and no launch of its own), four slices forward 2.6 -> 1.84 and back 1.87 -> 1.38 ms; the
 // three far fields and normal equations of 2,304 positions 2.7 -> 1.15 ms (the third field's columns end in the equations'
-// sums, which no field is written for).  Rows run at 4.6 TB/s, single columns at 4.5, limited by FP64 issue and LSU
-// wavefronts together.  Against the batched line transforms, which the generic variant, longer primes and sides up to 16 keep:
+// sums, which no field is written for).  Rows run at 4.6 TB/s, single columns at 4.5.  No unit is full: FP64 pipe 19 to 42 %,
+// LSU wavefronts 38 to 58, HBM 30 to 60; at 88 to 128 registers two CTAs fit an SM (22 % of its warps), and each one's phases
+// follow one another.  Against the batched line transforms, which the generic variant, longer primes and sides up to 16 keep:
 // four slices of 980 positions of 96 x 96 58 -> 17 ms per seven iterations, two mixed states of 1,035 14.9 -> 4.7 per six.
 #include <algorithm>
 #include <type_traits>

@@ -12,9 +12,9 @@
 // decimation in time of the any-size position pass (anypass.cuh): the fold writes the samples straight into
 // digit-reversed slots, and the last row stage writes natural order.
 //
-// Bound by shared-memory wavefronts (57 % of the pipe; FP64 pipe 28 %), the phases of one CTA in sequence.  Four samples'
+// Bound by shared-memory wavefronts (59 % of the pipe; FP64 pipe 26 %), the phases of one CTA in sequence.  Four samples'
 // fold loads in flight a thread and the spectrum's columns put in slot order once per table (scattered 16-byte reads took
-// 16 wavefronts a warp instead of 4) took the same table from 0.99 to 0.70 ms.  Before, each class took a ramp product, a
+// 16 wavefronts a warp instead of 4) took the same table from 0.99 to 0.68 ms.  Before, each class took a ramp product, a
 // batched line FFT through HBM in two passes, a scaling and a conversion: 2.05 ms, and one FP64 plane of scratch per
 // class (3,600 classes of 96 x 96: 1.93 -> 0.46 ms; 576 of 256 x 256: 1.37 -> 0.85 ms; the FP64 form at 128 x 128, which
 // ran the clustered plane kernel's inverse: 0.82 -> 0.76 ms).

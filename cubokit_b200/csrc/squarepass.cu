@@ -9,11 +9,11 @@
 // is known and a thread keeps its column (or row, or sample of a row) through a step.  The position's amplitudes are
 // prefetched into L2 when the CTA starts.
 //
-// Bound by latency between the barriers: issue about a third of the slots, shared memory a third of its wavefronts, so the
-// CTAs per SM decide (96 x 96: three of 384 threads at 56 registers 0.26 ms per pass of 3,600 positions, two at 80
-// registers 0.29; three of 192 threads 0.30; 64 x 64: four of 256 threads 0.109 ms, eight of 128 0.121).  They replace
-// register-resident line transforms, two CTAs per SM: 96 x 96 0.577 -> 0.258 ms (57 -> 129 Gpixel/s), 64 x 64 0.201 ->
-// 0.109 ms (73 -> 135).
+// Bound by shared-memory wavefronts (64 x 64 82 % of the pipe, 96 x 96 83 %; issue 62 and 51 %, HBM a quarter and a fifth).
+// Below that the CTAs per SM decide (before the projection's present form: 96 x 96 three of 384 threads at 56 registers 0.26
+// ms per pass of 3,600 positions, two at 80 registers 0.29, three of 192 threads 0.30; 64 x 64 four of 256 threads 0.109 ms,
+// eight of 128 0.121).  They replace register-resident line transforms, two CTAs per SM: 96 x 96 0.558 -> 0.240 ms (59 -> 138
+// Gpixel/s), 64 x 64 0.197 -> 0.087 (75 -> 170).
 #include "engine.h"
 #include "project.cuh"
 #include "regdft.cuh"
