@@ -726,7 +726,8 @@ void build_plan(cubo_ptycho_plan *p, const cubo_ptycho_problem *pr) {
     // kernel's build only, so the summation order (and the result) does not depend on the device
     const int kblocks = (n + 255) / 256;
     p->groups = std::max(1, std::min(P, 148 * probe_gather_resident_ctas<T>() / kblocks));
-    if (p->fast) p->groups = std::min(P, fast128_ctas());  // the position pass writes one partial per CTA
+    // the position pass writes one partial per CTA, as many as the first band has positions for
+    if (p->fast) p->groups = std::min(p->band_size, fast128_ctas());
     check(p->partial_grad.alloc((size_t)p->groups * n * sizeof(C2<T>)), "cudaMalloc");
     check(p->partial_weight.alloc((size_t)p->groups * n * sizeof(T)), "cudaMalloc");
     check(p->grad_p64.alloc((size_t)p->states * n * sizeof(double2)), "cudaMalloc");

@@ -124,3 +124,14 @@ def test_banded_fp32_iteration_equals_one_pass(monkeypatch):
     o1, p1, e1 = _bf16_run(s, 3, 0, monkeypatch, precision="fp32")
     ob, pb, eb = _bf16_run(s, 3, 148, monkeypatch, precision="fp32")
     assert np.array_equal(ob, o1) and np.array_equal(pb, p1) and np.array_equal(eb, e1)
+
+
+@pytest.mark.parametrize("band", [1, 16, 80])
+def test_banded_fp32_iteration_with_fewer_positions_than_ctas(monkeypatch, band):
+    """Bands smaller than the FP32 pass's 148 CTAs leave partials that no CTA writes: they are not summed.  The object of one
+    iteration has the same bits, the probe is grouped differently."""
+    s = scenes.raster_scene(scan=9, det=128, step=4, seed=29)
+    o1, p1, e1 = _bf16_run(s, 1, 0, monkeypatch, precision="fp32")
+    ob, pb, eb = _bf16_run(s, 1, band, monkeypatch, precision="fp32")
+    assert np.array_equal(ob, o1) and np.array_equal(eb, e1)
+    assert rel_l2(pb, p1) <= 1e-6, rel_l2(pb, p1)
